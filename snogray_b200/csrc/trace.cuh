@@ -231,7 +231,8 @@ __device__ __forceinline__ float4 *ring_slots() {
 // Each thread's current ray in shared memory, for the lanes that test its
 // list entries (a list round would otherwise move 14 values by shuffles):
 // uint4 k * kTraceBlock + threadIdx.x holds, for k = 0, 1, 2, (origin, t0),
-// (direction, t1) and the scene's list-record pointer.
+// (direction, t1) and the scene's list-record pointer in x, y; z, w of the
+// third belong to the list round: what the units of the warp's k-th owner need.
 __device__ __forceinline__ uint4 *ray_slots() {
   __shared__ uint4 rays[3 * kTraceBlock];
   return rays;
@@ -332,7 +333,7 @@ struct Traversal {
       slot[0] = make_uint4(__float_as_uint(o.x), __float_as_uint(o.y), __float_as_uint(o.z), __float_as_uint(t0_));
       slot[kTraceBlock] =
           make_uint4(__float_as_uint(d.x), __float_as_uint(d.y), __float_as_uint(d.z), __float_as_uint(t1_));
-      slot[2 * kTraceBlock] = make_uint4(uint32_t(pl), uint32_t(pl >> 32), 0u, 0u);
+      reinterpret_cast<uint2 *>(slot + 2 * kTraceBlock)[0] = make_uint2(uint32_t(pl), uint32_t(pl >> 32));
     }
     // 1 / d rounded once, as the reference's division (__frcp_rn is the
     // correctly rounded reciprocal, the same value as 1.0f / d).
@@ -532,20 +533,6 @@ struct Traversal {
   }
 };
 
-// Position of the K-th (1-based) set bit of MASK; MASK has at least K bits set.
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t mask, uint32_t k) {
-  uint32_t p = 0;
-#pragma unroll
-  for (uint32_t w = 16; w >= 1; w >>= 1) {
-    const uint32_t c = __popc((mask >> p) & ((1u << w) - 1u));   // set bits in [p, p + w)
-    if (c < k) {
-      k -= c;
-      p += w;
-    }
-  }
-  return p;
-}
-
 // One warp-cooperative round of list tests.  Every lane with a list pending
 // (WANT) owns the next entries of its list; the warp's pending entries, in
 // lane order and list order, are dealt to its 32 lanes (one or two
@@ -568,12 +555,18 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t mask, uint32_t k) {
 // probe found long lists along rays (SceneImpl's pair_lists: 8 % faster on
 // a 2M-triangle soup, 3 % slower on the terrain, whose lists are short).
 // Any-hit rounds deal single entries: a walk stops at its first hit.
+//
+// Bookkeeping.  An owner's units are consecutive lanes [excl, excl + np), so
+// one ballot of the hits gives every owner its own hits by a mask; the few
+// that hit are compared in a loop over each owner's hits (most often none or
+// one).  The k-th owner leaves what its units need in the warp's k-th ray
+// slot, where a unit finds it by counting the first units at or before its
+// lane.
 template <int STACK, int ANY = kMixed, int PER = (ANY == kMixed ? 2 : 1)>
 __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool any, TraceCounters &cnt) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr uint32_t kPer = uint32_t(PER);
   const uint32_t lane = threadIdx.x & 31u;
-  __syncwarp();   // the warp's ray-slot writes (new rays, shrunk t1) are visible
   uint32_t c = want ? tr.lend - tr.lp : 0u;
   c = c < 32u * kPer ? c : 32u * kPer;
   const uint32_t np = (c + kPer - 1u) / kPer;   // dealt units: pairs (or entries)
@@ -584,64 +577,45 @@ __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool
     if (lane >= uint32_t(off)) incl += v;
   }
   const uint32_t excl = incl - np;
-  const bool owner = np > 0u && excl < 32u;
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   if (total == 0u) return false;
-  const bool item = lane < total;
-  // The owner of the unit at this lane's position.
-  uint32_t own = lane;
-  if (ANY == kAnyOnly) {
-    // The k-th owner, k the owners whose first unit lies at or before the
-    // position.
-    const uint32_t owners = __ballot_sync(kFull, owner);
-    const uint32_t starts = __reduce_or_sync(kFull, owner ? (1u << excl) : 0u);
-    const uint32_t upto = lane == 31u ? kFull : ((2u << lane) - 1u);
-    if (item) own = nth_set_bit(owners, uint32_t(__popc(starts & upto)));
-  } else {
-    // The first lane whose inclusive count exceeds the position (the counts
-    // never decrease with the lane): a binary search of five shuffles.
-    // Fewer instructions than the bit search above (the closest-hit kernel
-    // 2 % faster on the terrain frame), but a longer chain of dependent
-    // latencies, which the any-hit kernel's frequent sparse rounds feel (2 %
-    // slower with it).
-    uint32_t first = 0u;
-#pragma unroll
-    for (uint32_t w = 16u; w >= 1u; w >>= 1) {
-      const uint32_t v = __shfl_sync(kFull, incl, first + w - 1u);
-      first += v <= lane ? w : 0u;
-    }
-    if (item) own = first;
+  const bool owner = np > 0u && excl < 32u;
+  const uint32_t owners = __ballot_sync(kFull, owner);
+  const uint32_t starts = __reduce_or_sync(kFull, owner ? (1u << excl) : 0u);
+  uint4 *const wslot = ray_slots() + (threadIdx.x & ~31u);
+  if (owner) {
+    // First entry of a unit at lane l: base + kPer * l; entries end at base + stop.
+    const uint32_t k = __popc(owners & ((1u << lane) - 1u));
+    reinterpret_cast<uint2 *>(wslot + 2 * kTraceBlock + k)[1] =
+        make_uint2(tr.lp - kPer * excl, lane | (any ? 32u : 0u) | ((kPer * excl + c) << 8));
   }
-  // The owner's ray and list.
-  const uint32_t o_excl = __shfl_sync(kFull, excl, own);
-  const uint32_t o_lp = __shfl_sync(kFull, tr.lp, own);
-  const uint32_t o_c = __shfl_sync(kFull, c, own);
-  const bool o_any = ANY != kClosestOnly && ((__ballot_sync(kFull, any) >> own) & 1u) != 0u;
+  __syncwarp();   // these, and the warp's ray-slot writes (new rays, shrunk t1), are visible
   uint32_t pid = PREF_END, which = 0u;
   bool hit = false;
   float th = 0.f;
-  if (item) {
-    const uint4 *slot = ray_slots() + ((threadIdx.x & ~31u) + own);
+  if (lane < total) {
+    const uint32_t k = __popc(starts & (kFull >> (31u - lane))) - 1u;
+    const uint2 unit = reinterpret_cast<const uint2 *>(wslot + 2 * kTraceBlock + k)[1];
+    const uint4 *slot = wslot + (unit.y & 31u);
     const uint4 ra = slot[0], rb = slot[kTraceBlock];
+    const uint2 rc = reinterpret_cast<const uint2 *>(slot + 2 * kTraceBlock)[0];
     const float3 ro = f3(__uint_as_float(ra.x), __uint_as_float(ra.y), __uint_as_float(ra.z));
     const float3 rd = f3(__uint_as_float(rb.x), __uint_as_float(rb.y), __uint_as_float(rb.z));
     const float rt0 = __uint_as_float(ra.w);
     const float rt1 = __uint_as_float(rb.w);
-    const uint4 rc = slot[2 * kTraceBlock];
     // The entries' primitive records from the owner's scene's list records.
     const unsigned long long o_lrec = (unsigned long long)rc.x | ((unsigned long long)rc.y << 32);
-    const uint32_t k0 = kPer * (lane - o_excl);   // the first entry's index in the owner's round
-    const float4 *p = reinterpret_cast<const float4 *>(o_lrec) + 3 * size_t(o_lp + k0);
+    const float4 *p = reinterpret_cast<const float4 *>(o_lrec) + 3 * size_t(unit.x + kPer * lane);
     const PrimRec r0{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
     th = rt1;
     hit = test_prim<ANY != kAnyOnly>(r0, ro, rd, rt0, th);
     pid = __float_as_uint(r0.c.w);
-    if (kPer == 2u && k0 + 1u < o_c && !(hit && o_any)) {
+    if (kPer == 2u && kPer * lane + 1u < (unit.y >> 8) && !(ANY != kClosestOnly && hit && (unit.y & 32u))) {
       const PrimRec r1{__ldg(p + 3), __ldg(p + 4), __ldg(p + 5)};
       float th1 = rt1;
       const bool hit1 = test_prim<ANY != kAnyOnly>(r1, ro, rd, rt0, th1);
       // The later entry wins only with a smaller t (the earlier one keeps ties).
-      if (hit1 && (!hit || __float_as_uint(th1) < __float_as_uint(th))) {
+      if (hit1 && (!hit || th1 < th)) {
         hit = true;
         th = th1;
         pid = __float_as_uint(r1.c.w);
@@ -649,32 +623,46 @@ __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool
       }
     }
   }
-  // Reduce over each owner's units (positive t: its bits order like the value).
-  const unsigned grp = __match_any_sync(kFull, item ? own : 32u + lane);
-  const uint32_t tb = hit ? __float_as_uint(th) : kFull;
-  const uint32_t tmin = __reduce_min_sync(grp, tb);
-  const uint32_t best = __reduce_min_sync(grp, (hit && (o_any || tb == tmin)) ? lane : kFull);
-  // Each owner reads the result at its first unit's lane.
-  const uint32_t b = __shfl_sync(kFull, best, owner ? excl : lane);
-  const uint32_t src = b < 32u ? b : lane;
-  const uint32_t b_pid = __shfl_sync(kFull, pid, src);
-  const float b_t = __shfl_sync(kFull, th, src);
-  const uint32_t b_which = __shfl_sync(kFull, which, src);
-  if (!owner) return false;
-  const uint32_t room = kPer * (32u - excl);
-  const uint32_t used = c < room ? c : room;
-  if (b < 32u) {
-    tr.hit_ref = b_pid;
-    if (any) {
-      cnt.tests += kPer * (b - excl) + b_which + 1u;
-      tr.lp = tr.lend;
-      return true;
+  const uint32_t hits = __ballot_sync(kFull, hit);
+  const uint32_t room = 32u - excl;   // (excl > 31 only where !owner)
+  uint32_t mine = owner ? hits & ((np < room ? (1u << np) - 1u : kFull) << excl) : 0u;
+  bool over = false;
+  if (hits) {   // the same for the whole warp
+    const bool found = mine != 0u;
+    uint32_t best = found ? uint32_t(__ffs(mine)) - 1u : lane;
+    float b_t = __shfl_sync(kFull, th, best);
+    if (ANY != kAnyOnly) {
+      if (ANY == kMixed && any) mine = 0u;   // the earliest stands
+      mine &= mine - 1u;
+      while (__any_sync(kFull, mine != 0u)) {
+        const uint32_t src = mine ? uint32_t(__ffs(mine)) - 1u : lane;
+        const float t = __shfl_sync(kFull, th, src);
+        if (mine && t < b_t) {
+          b_t = t;
+          best = src;
+        }
+        mine &= mine - 1u;
+      }
     }
-    tr.set_t1(b_t);
+    const uint32_t b_pid = __shfl_sync(kFull, pid, best);
+    const uint32_t b_which = kPer == 2u && ANY != kClosestOnly ? __shfl_sync(kFull, which, best) : 0u;
+    if (found) {
+      tr.hit_ref = b_pid;
+      if (ANY != kClosestOnly && any) {
+        cnt.tests += kPer * (best - excl) + b_which + 1u;
+        tr.lp = tr.lend;
+        over = true;
+      } else {
+        tr.set_t1(b_t);
+      }
+    }
   }
-  cnt.tests += used;
-  tr.lp += used;
-  return false;
+  if (owner && !over) {
+    const uint32_t used = c < kPer * room ? c : kPer * room;
+    cnt.tests += used;
+    tr.lp += used;
+  }
+  return over;
 }
 
 // Rays a warp takes per refill: 32 (one per lane) keeps the launch's tail
