@@ -176,7 +176,9 @@ cudaError_t launch_trace_batch(const DevScene &s, const float *rays, uint32_t n,
                                uint32_t *err, uint32_t *fetch, cudaStream_t st, int *launches) {
   if (n == 0) return cudaSuccess;
   const int threads = kTraceBlock;
-  const uint32_t want = (n + threads - 1) / threads;
+  // A warp per ray while the resident grid has them: a small batch takes as
+  // long as its slowest warp (RayDispenser).
+  const uint32_t want = n / (threads / 32) + (n % (threads / 32) ? 1u : 0u);
   auto grid = [&](uint32_t resident) { return want < resident ? want : resident; };
   switch (stack_class_for_depth(s.max_depth)) {
     case 32: k_trace_batch<32><<<grid(resident_grid(k_trace_batch<32>, threads)), threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err, fetch); break;

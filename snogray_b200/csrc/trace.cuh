@@ -561,7 +561,9 @@ struct Traversal {
 // that hit are compared in a loop over each owner's hits (most often none or
 // one).  The k-th owner leaves what its units need in the warp's k-th ray
 // slot, where a unit finds it by counting the first units at or before its
-// lane.
+// lane.  (Against a match over the owners, two reductions per owner's group
+// and a five-shuffle search per unit: terrain frame 273.3 -> 225.5 ms, 16M
+// rays in 1M triangles 24.7 -> 20.15 ms.)
 template <int STACK, int ANY = kMixed, int PER = (ANY == kMixed ? 2 : 1)>
 __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool any, TraceCounters &cnt) {
   constexpr unsigned kFull = 0xffffffffu;
@@ -665,13 +667,6 @@ __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool
   return over;
 }
 
-// Rays a warp takes per refill: 32 (one per lane) keeps the launch's tail
-// short -- 32 rather than 64 measured 1.4 % faster on the terrain frame, 16 in
-// between.
-#ifndef SNOG_DISPENSE_CHUNK
-#define SNOG_DISPENSE_CHUNK 32
-#endif
-
 // Idle lanes a warp gathers before it refills them (1 = refill at once).
 #ifndef SNOG_REFILL_MIN
 #define SNOG_REFILL_MIN 4
@@ -689,14 +684,29 @@ constexpr uint32_t kRoundMin = SNOG_ROUND_MIN;
 static_assert(kRoundMin >= 1u && kRoundMin <= 32u, "closest-hit round threshold must not exceed the node-step cut");
 
 // Warp-cooperative ray dispenser for the persistent trace kernels: lanes
-// whose ray is finished take the next index from a warp-local range of CHUNK
-// rays, refilled with one atomic on the launch's counter.  All 32 lanes of
+// whose ray is finished take the next index from a warp-local range of up to
+// 32 rays, refilled with one atomic on the launch's counter.  All 32 lanes of
 // the warp must call fetch() together.
+//
+// A launch lasts as long as its slowest warp, and a warp with few rays runs
+// through their lists faster than one with 32 (its list rounds are shared by
+// fewer rays).  So a launch with fewer rays than lanes spreads them: each warp
+// holds at most its even share, LIMIT of 1 to 32 rays, in its first LIMIT
+// lanes.  999 rays among 10k triangles 147 -> 99 us, a 64x48 Cornell render
+// 803 -> 621 us, the late bounces of an 853x479 terrain render 12.5 -> 11.6
+// ms; launches with 32 rays a warp are unchanged (ranges that shrink with the
+// rays left, besides, measured 1-2 % slower there).
 struct RayDispenser {
-  static constexpr uint32_t kChunk = SNOG_DISPENSE_CHUNK;
   static constexpr uint32_t kIdle = 0xffffffffu;
   uint32_t next = 0, end = 0;
+  uint32_t limit;
   bool exhausted = false;
+
+  __device__ __forceinline__ explicit RayDispenser(uint32_t n) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t share = n / warps + (n % warps ? 1u : 0u);
+    limit = share < 1u ? 1u : share < 32u ? share : 32u;
+  }
 
   // Returns the new ray index for a lane that asked (NEED) and got one,
   // else kIdle.  Sets *all_idle when every lane is idle and no rays remain.
@@ -708,13 +718,13 @@ struct RayDispenser {
     if (mask) {
       if (next >= end && !exhausted) {
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(counter, kChunk);
+        if (lane == 0) base = atomicAdd(counter, limit);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= n) {
           exhausted = true;
         } else {
           next = base;
-          end = base + kChunk < n ? base + kChunk : n;
+          end = base + limit < n ? base + limit : n;
         }
       }
       const uint32_t rank = __popc(mask & ((1u << lane) - 1u));
@@ -741,7 +751,9 @@ __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, Trac
   StackRec stk[Traversal<STACK>::kRecs];
   Traversal<STACK> tr;
   tr.stk = stk;
-  RayDispenser disp;
+  RayDispenser disp(n);
+  const bool takes = (threadIdx.x & 31u) < disp.limit;
+  const uint32_t refill_min = kRefillMin < disp.limit ? kRefillMin : disp.limit;
   uint32_t ray = RayDispenser::kIdle;
   bool any = false;
   for (;;) {
@@ -749,8 +761,8 @@ __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, Trac
     // Idle lanes take new rays only once kRefillMin of them are idle: a ray
     // start (queue loads, root slab set-up, ray slot) then runs on several
     // lanes at once instead of on one or two every iteration.
-    const uint32_t idle_lanes = __popc(__ballot_sync(0xffffffffu, ray == RayDispenser::kIdle));
-    const bool need = ray == RayDispenser::kIdle && idle_lanes >= kRefillMin;
+    const uint32_t idle_lanes = __popc(__ballot_sync(0xffffffffu, takes && ray == RayDispenser::kIdle));
+    const bool need = takes && ray == RayDispenser::kIdle && idle_lanes >= refill_min;
     const uint32_t got = disp.fetch(dispenser, n, need, ray != RayDispenser::kIdle, &all_idle);
     if (all_idle) break;
     if (got != RayDispenser::kIdle) {
