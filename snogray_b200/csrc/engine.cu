@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_closest
   const uint32_t n = ctl->qcount[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->rays_closest += n;
   TraceCounters c{0, 0, 0};
-  trace_loop<STACK, kClosestOnly, PER>(
+  trace_loop<STACK, kClosestOnly, PER, false>(
       &ctl->disp_closest, n, c,
       [&](uint32_t ray, Traversal<STACK> &tr, bool &any) {
         const float4 o = q.o[ray], d = q.d[ray];
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_shadow(
   const uint32_t n = ctl->scount;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->rays_shadow += n;
   TraceCounters c{0, 0, 0};
-  trace_loop<STACK, kAnyOnly>(
+  trace_loop<STACK, kAnyOnly, 1, false>(
       &ctl->disp_shadow, n, c,
       [&](uint32_t ray, Traversal<STACK> &tr, bool &any) {
         const float4 o = q.o[ray], d = q.d[ray];

@@ -298,6 +298,7 @@ __global__ void k_oct_finish_nodes(uint4 *nodes, const uint32_t *blen, const uin
       r.x = 0;
       leaves++;
     }
+    r.y = child_masks(r.y);
     r.z = blen[b] ? 4u + boff[b] : 0u;
     r.w = blen[b];
     nodes[b] = r;

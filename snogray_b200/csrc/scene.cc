@@ -136,6 +136,7 @@ std::vector<uint4> compact_nodes(const OctreeArrays &o, std::vector<uint32_t> &p
         expect++;
         r.y |= 1u << s;
       }
+      r.y = child_masks(r.y);
     }
     if (r.z) {
       const uint32_t start = uint32_t(plist4.size());

@@ -90,8 +90,19 @@ struct DevMedium {
 // order, so the eight child ids of the reference's node
 // (space/octree-node.h:27-86) reduce to the first child's id and an 8-bit
 // mask: child(slot) = first + popc(mask & ((1 << slot) - 1)).
-//   x = first child id, y = child mask (0 = leaf),
+//   x = first child id, y = child masks (0 = leaf),
 //   z = first entry of the surface list in plist, w = list length
+// The low byte of y is that mask; byte k holds it with the octant bits of k
+// (z = 1, y = 2) flipped, so that a walk of a ray into octant o finds the
+// children by their place along the ray in byte o & 3, with the halves of the
+// byte exchanged for o & 4.
+SNOG_HD uint32_t child_masks(uint32_t m) {
+  const uint32_t z = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
+  const uint32_t y = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
+  const uint32_t yz = ((z & 0x33u) << 2) | ((z >> 2) & 0x33u);
+  return m | (z << 8) | (y << 16) | (yz << 24);
+}
+
 struct DevScene {
   const uint4 *nodes;
   const uint32_t *plist;

@@ -22,7 +22,7 @@ namespace snog {
 #define SNOG_TRACE_BATCH_MINBLOCKS 7
 #endif
 
-template <int STACK>
+template <int STACK, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_BATCH_MINBLOCKS) k_trace_batch(DevScene s, const float *__restrict__ rays,
                                                      uint32_t n, uint32_t n_closest,
                                                      int32_t *__restrict__ prim, float *__restrict__ tout,
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_BATCH_MINBLOCKS) k_tra
             f3(rays[3 * size_t(n) + ray], rays[4 * size_t(n) + ray], rays[5 * size_t(n) + ray]), 0.f,
             rays[6 * size_t(n) + ray]);
     any = ray >= n_closest;
-    base = c;
+    if (COUNT) base = c;
   };
   auto done = [&](uint32_t i, Traversal<STACK> &tr, bool any) {
     const bool closest = !any;
@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_BATCH_MINBLOCKS) k_tra
       nrm[3 * size_t(i) + 1] = nv.y;
       nrm[3 * size_t(i) + 2] = nv.z;
     }
+    if (!COUNT) return;
     if (closest) {
       cn += c.nodes - base.nodes;
       ct += c.tests - base.tests;
@@ -73,9 +74,9 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_BATCH_MINBLOCKS) k_tra
       at += c.tests - base.tests;
     }
   };
-  trace_loop<STACK>(fetch, n, c, start, done);
+  trace_loop<STACK, kMixed, 2, COUNT>(fetch, n, c, start, done);
   if (c.overflow) atomicOr(err, 1u);
-  if (counters) {
+  if (COUNT) {
     // All lanes reach this point: reduce per warp, one atomic per warp.
     for (int off = 16; off > 0; off >>= 1) {
       cn += __shfl_down_sync(0xffffffffu, cn, off);
@@ -179,12 +180,16 @@ cudaError_t launch_trace_batch(const DevScene &s, const float *rays, uint32_t n,
   // A warp per ray while the resident grid has them: a small batch takes as
   // long as its slowest warp (RayDispenser).
   const uint32_t want = n / (threads / 32) + (n % (threads / 32) ? 1u : 0u);
-  auto grid = [&](uint32_t resident) { return want < resident ? want : resident; };
+  auto launch = [&](auto kernel) {
+    const uint32_t resident = resident_grid(kernel, threads);
+    kernel<<<want < resident ? want : resident, threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err,
+                                                                  fetch);
+  };
   switch (stack_class_for_depth(s.max_depth)) {
-    case 32: k_trace_batch<32><<<grid(resident_grid(k_trace_batch<32>, threads)), threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err, fetch); break;
-    case 64: k_trace_batch<64><<<grid(resident_grid(k_trace_batch<64>, threads)), threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err, fetch); break;
-    case 128: k_trace_batch<128><<<grid(resident_grid(k_trace_batch<128>, threads)), threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err, fetch); break;
-    case 256: k_trace_batch<256><<<grid(resident_grid(k_trace_batch<256>, threads)), threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err, fetch); break;
+    case 32: counters ? launch(k_trace_batch<32, true>) : launch(k_trace_batch<32, false>); break;
+    case 64: counters ? launch(k_trace_batch<64, true>) : launch(k_trace_batch<64, false>); break;
+    case 128: counters ? launch(k_trace_batch<128, true>) : launch(k_trace_batch<128, false>); break;
+    case 256: counters ? launch(k_trace_batch<256, true>) : launch(k_trace_batch<256, false>); break;
     default: return cudaErrorInvalidValue;
   }
   if (launches) (*launches)++;

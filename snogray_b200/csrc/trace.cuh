@@ -193,13 +193,12 @@ __device__ __forceinline__ bool test_prim(const PrimRec &r, float3 o, float3 d, 
 // The pending children of one visited node, as one stack record: the
 // node's near-half lower bounds, midpoints and far-half upper bounds (every
 // child's slab bounds are a selection of these, per axis), its first child's
-// index, its child mask and the visiting positions of the children not yet
-// entered.  One record per visited node with two or more qualifying children,
+// index, its child mask and the children not yet entered (by octant bits).  One record per visited node with two or more qualifying children,
 // instead of one entry per waiting child: a visit pushes at most once, and
 // the stack holds at most one record per tree level.
 struct StackRec {
   float4 a;   // near_lo.xyz, first child index
-  float4 b;   // mid.xyz, child mask | visiting positions still to enter << 8
+  float4 b;   // mid.xyz, child mask | children still to enter << 8
   float4 c;   // far.xyz
 };
 
@@ -268,9 +267,12 @@ __device__ __forceinline__ bool gate_open(uint32_t cb, float t0, float t1, float
   return gx && gy && gz;
 }
 
-// Octant bits (x = 4, y = 2, z = 1) of the I-th child in the reference's
-// visiting order 0,1,2,4,3,5,6,7 (before the xor with the ray's octant).
-__device__ __forceinline__ uint32_t visit_bits(uint32_t i) { return i == 3u ? 4u : i == 4u ? 3u : i; }
+// The child of the waiting set VM (bit cb = the child with octant bits cb,
+// x = 4, y = 2, z = 1, a set bit meaning the half the ray enters later) that
+// the reference visits first: its order is 0,1,2,4,3,5,6,7, so 4 goes before 3.
+__device__ __forceinline__ uint32_t first_child(uint32_t vm) {
+  return (vm & 0x1fu) == 0x18u ? 4u : uint32_t(__ffs(vm)) - 1u;
+}
 
 // A resumable octree walk for one ray.  init() sets up the root's slab
 // bounds (space/octree.cc:119-135); node_step() processes one octree entry --
@@ -413,15 +415,14 @@ struct Traversal {
                  rc = r[(3 * pos + 2) * kTraceBlock];
     const uint32_t bits = __float_as_uint(rb.w);
     const uint32_t vm = bits >> 8;
-    const uint32_t i = __ffs(vm) - 1u;   // the earliest visiting position left
-    const uint32_t rest = vm & (vm - 1u);
+    const uint32_t cb = first_child(vm);
+    const uint32_t rest = vm & ~(1u << cb);
     if (rest) {
       reinterpret_cast<uint32_t *>(r + (3 * pos + 1) * kTraceBlock)[3] = (bits & 0xffu) | (rest << 8);
       ring = base | (n << 4);
     } else {
       ring = n > 1u ? (base | ((n - 1u) << 4)) : 0u;   // an emptied ring restarts at position 0
     }
-    const uint32_t cb = visit_bits(i);
     const uint32_t slot = cb ^ (octant & 7u);
     node = __float_as_uint(ra.w) + __popc(bits & 0xffu & ((1u << slot) - 1u));
     gate = cb | kGateFlag;
@@ -441,22 +442,25 @@ struct Traversal {
   // the tests and their order are the reference's.
   // ANY: the queries the calling kernel runs -- kClosestOnly, kAnyOnly or
   // kMixed (checked per ray) -- so closest-hit kernels carry no any-hit branch.
-  template <bool FAST = true, int ANY = kMixed>
+  // COUNT: node calls are counted.
+  template <int ANY, bool COUNT>
   __device__ __forceinline__ void node_step(TraceCounters &cnt) {
     if (!have && !pop()) return;
     have = false;
-    const bool slow = !FAST || (octant & kSlowSlab);
+    const bool slow = octant & kSlowSlab;
     bool open = true;
     const bool any_query = ANY == kAnyOnly || (ANY == kMixed && (octant & kAnyHit));
     if ((gate & kGateFlag) && any_query) {
       // An any-hit query's extent never changes, so an entry with a parent
       // gate passed the very gate and cull it would be given now when it
       // was pushed (or entered): the call happens and the node is open.
-      cnt.nodes++;
+      if (COUNT) cnt.nodes++;
     } else {
-      if (gate & kGateFlag) open = gate_open(gate & 7u, t0, t1, lo, hi);
+      // The cull decides alone where bounds are finite: it closes whatever the
+      // gate does.  The gate is where a call is counted.
+      if ((COUNT || slow) && (gate & kGateFlag)) open = gate_open(gate & 7u, t0, t1, lo, hi);
       if (open) {
-        cnt.nodes++;
+        if (COUNT) cnt.nodes++;
         open = slow ? slab_open(t0, t1, lo, hi) : slab_open_finite(t0, t1, lo, hi);
       }
       if (!open) return;
@@ -473,61 +477,58 @@ struct Traversal {
     // the same rounded sums as the reference's child ranges.
     const float3 mid = f3(__fadd_rn(lo.x, half.x), __fadd_rn(lo.y, half.y), __fadd_rn(lo.z, half.z));
     const float3 far = f3(__fadd_rn(mid.x, half.x), __fadd_rn(mid.y, half.y), __fadd_rn(mid.z, half.z));
-    const float3 near_lo = f3(__fadd_rn(lo.x, 0.f), __fadd_rn(lo.y, 0.f), __fadd_rn(lo.z, 0.f));
-    // Which children pass gate and cull, by visiting position (bit i).  At
-    // most 4 pass: one octant per crossing of each of the three midplanes.
+    // Which children pass gate and cull, by octant bits.  At most 4 pass: one
+    // octant per crossing of each of the three midplanes.
     const uint32_t oct = octant & 7u;
     uint32_t vm = 0;
     if (slow) {
 #pragma unroll
-      for (uint32_t i = 0; i < 8; i++) {
-        const uint32_t cb = visit_bits(i);
-        const uint32_t slot = cb ^ oct;
-        const float3 clo = f3((cb & 4) ? mid.x : near_lo.x, (cb & 2) ? mid.y : near_lo.y,
-                              (cb & 1) ? mid.z : near_lo.z);
+      for (uint32_t cb = 0; cb < 8; cb++) {
+        const float3 clo = f3((cb & 4) ? mid.x : lo.x, (cb & 2) ? mid.y : lo.y, (cb & 1) ? mid.z : lo.z);
         const float3 chi = f3((cb & 4) ? far.x : mid.x, (cb & 2) ? far.y : mid.y, (cb & 1) ? far.z : mid.z);
-        const bool ok = ((nd.y >> slot) & 1u) & gate_open(cb, t0, t1, clo, chi) & slab_open(t0, t1, clo, chi);
-        vm |= ok ? (1u << i) : 0u;
+        const bool ok = ((nd.y >> (cb ^ oct)) & 1u) & gate_open(cb, t0, t1, clo, chi) & slab_open(t0, t1, clo, chi);
+        vm |= ok ? (1u << cb) : 0u;
       }
     } else {
-      // The same tests from shared pieces: per axis the near and far halves'
-      // gates, and the child's entry max(t0, lo.x, lo.y, lo.z) and exit
-      // min(t1, hi.x, hi.y, hi.z) built from an x part and a yz part.  The
-      // pieces are scalars picked by selects, not small arrays: an array
-      // indexed in the loop may be placed in local memory, which a node visit
-      // would then write and read a dozen times.
-      const bool gx0 = t0 < mid.x, gx1 = t1 > mid.x, gy0 = t0 < mid.y, gy1 = t1 > mid.y, gz0 = t0 < mid.z,
-                 gz1 = t1 > mid.z;
-      const float in_x0 = fmaxf(t0, near_lo.x), in_x1 = fmaxf(t0, mid.x);
-      const float out_x0 = fminf(t1, mid.x), out_x1 = fminf(t1, far.x);
-      const float in_yz00 = fmaxf(near_lo.y, near_lo.z), in_yz01 = fmaxf(near_lo.y, mid.z),
-                  in_yz10 = fmaxf(mid.y, near_lo.z), in_yz11 = fmaxf(mid.y, mid.z);
-      const float out_yz00 = fminf(mid.y, mid.z), out_yz01 = fminf(mid.y, far.z), out_yz10 = fminf(far.y, mid.z),
-                  out_yz11 = fminf(far.y, far.z);
-#pragma unroll
-      for (uint32_t i = 0; i < 8; i++) {
-        const uint32_t cb = visit_bits(i);
-        const bool bx = (cb & 4u) != 0u, by = (cb & 2u) != 0u, bz = (cb & 1u) != 0u;
-        const uint32_t slot = cb ^ oct;
-        const float in_yz = by ? (bz ? in_yz11 : in_yz10) : (bz ? in_yz01 : in_yz00);
-        const float out_yz = by ? (bz ? out_yz11 : out_yz10) : (bz ? out_yz01 : out_yz00);
-        const bool ok = ((nd.y >> slot) & 1u) && (bx ? gx1 : gx0) && (by ? gy1 : gy0) && (bz ? gz1 : gz0) &&
-                        (fmaxf(bx ? in_x1 : in_x0, in_yz) < fminf(bx ? out_x1 : out_x0, out_yz));
-        vm |= ok ? (1u << i) : 0u;
-      }
+      // The same tests taken apart.  lo <= mid <= far per axis (half is not
+      // negative where the node is open), so a child's entry is the largest
+      // of ENTRY and the midpoints of its far axes, its exit the smallest of
+      // EXIT and the midpoints of its near axes, and entry < exit holds
+      // exactly when each of the former is below each of the latter: a far
+      // axis' midpoint below EXIT, a near one's above ENTRY, and a far axis'
+      // midpoint below a near one's.  Each failed comparison takes its
+      // children out of the mask.  The gates follow from the same
+      // comparisons.  (Against a maximum, a minimum and four gates for each of
+      // eight children: terrain frame 224.5 -> 201.8 ms, 16M rays in 1M
+      // triangles 20.2 -> 17.6 ms, with the uncounted cull above.)
+      const float entry = fmaxf(fmaxf(t0, lo.x), fmaxf(lo.y, lo.z));
+      const float exit = fminf(fminf(t1, far.x), fminf(far.y, far.z));
+      vm = (__byte_perm(nd.y, 0u, (oct & 3u) * 0x1111u) >> (oct & 4u)) & 0xffu;   // children that exist
+      if (!(entry < exit)) vm = 0u;
+      if (!(entry < mid.x)) vm &= 0xf0u;
+      if (!(entry < mid.y)) vm &= 0xccu;
+      if (!(entry < mid.z)) vm &= 0xaau;
+      if (!(mid.x < exit)) vm &= 0x0fu;
+      if (!(mid.y < exit)) vm &= 0x33u;
+      if (!(mid.z < exit)) vm &= 0x55u;
+      if (!(mid.x < mid.y)) vm &= ~0x30u;   // x far, y near
+      if (!(mid.y < mid.x)) vm &= ~0x0cu;
+      if (!(mid.x < mid.z)) vm &= ~0x50u;   // x far, z near
+      if (!(mid.z < mid.x)) vm &= ~0x0au;
+      if (!(mid.y < mid.z)) vm &= ~0x44u;   // y far, z near
+      if (!(mid.z < mid.y)) vm &= ~0x22u;
     }
     if (!vm) return;
     // The first qualifying child becomes the current entry; the others wait
     // in one record and are entered in visiting order after the first
     // child's subtree (pop), as the reference's loop over the children does.
-    const uint32_t rest = vm & (vm - 1u);
-    if (rest) push(near_lo, mid, far, nd.x, (nd.y & 0xffu) | (rest << 8), cnt);
-    const uint32_t i = __ffs(vm) - 1u;
-    const uint32_t cb = visit_bits(i);
+    const uint32_t cb = first_child(vm);
+    const uint32_t rest = vm & ~(1u << cb);
+    if (rest) push(lo, mid, far, nd.x, (nd.y & 0xffu) | (rest << 8), cnt);
     const uint32_t slot = cb ^ oct;
     node = nd.x + __popc(nd.y & ((1u << slot) - 1u));
     gate = cb | kGateFlag;
-    lo = f3((cb & 4) ? mid.x : near_lo.x, (cb & 2) ? mid.y : near_lo.y, (cb & 1) ? mid.z : near_lo.z);
+    lo = f3((cb & 4) ? mid.x : lo.x, (cb & 2) ? mid.y : lo.y, (cb & 1) ? mid.z : lo.z);
     hi = f3((cb & 4) ? far.x : mid.x, (cb & 2) ? far.y : mid.y, (cb & 1) ? far.z : mid.z);
     have = true;
   }
@@ -564,7 +565,7 @@ struct Traversal {
 // lane.  (Against a match over the owners, two reductions per owner's group
 // and a five-shuffle search per unit: terrain frame 273.3 -> 225.5 ms, 16M
 // rays in 1M triangles 24.7 -> 20.15 ms.)
-template <int STACK, int ANY = kMixed, int PER = (ANY == kMixed ? 2 : 1)>
+template <int STACK, int ANY, int PER>
 __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool any, TraceCounters &cnt) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr uint32_t kPer = uint32_t(PER);
@@ -745,7 +746,7 @@ struct RayDispenser {
 // round of list entries pending, every live lane without a list pending
 // visits one octree entry; then the warp tests one round of pending list
 // entries together.  All 32 lanes of every warp must run it.
-template <int STACK, int ANY = kMixed, int PER = (ANY == kMixed ? 2 : 1), class Start, class Done>
+template <int STACK, int ANY, int PER, bool COUNT, class Start, class Done>
 __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, TraceCounters &cnt, Start start,
                                            Done done) {
   StackRec stk[Traversal<STACK>::kRecs];
@@ -775,7 +776,7 @@ __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, Trac
     // a round: list rounds run full, node steps run with more lanes at once.
     const uint32_t pend = (busy && tr.lp < tr.lend) ? tr.lend - tr.lp : 0u;
     const uint32_t pending = __reduce_add_sync(0xffffffffu, pend < 32u ? pend : 32u);
-    if (pending < 32u && busy && tr.lp >= tr.lend && !tr.finished()) tr.template node_step<true, ANY>(cnt);
+    if (pending < 32u && busy && tr.lp >= tr.lend && !tr.finished()) tr.template node_step<ANY, COUNT>(cnt);
     // Closest-hit kernels test lists only once at least kRoundMin entries
     // are pending, unless no lane could visit a node: fewer, fuller rounds
     // (2 % off the terrain frame; the any-hit and mixed kernels, whose

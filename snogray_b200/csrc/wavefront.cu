@@ -30,6 +30,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "launch.h"
 #include "pathstate.cuh"
@@ -109,10 +110,10 @@ __device__ __forceinline__ void warp_count(unsigned long long *p, unsigned long 
 // Persistent closest-hit kernel: warps take rays from the queue through a
 // RayDispenser (counters[4]) and interleave one octree entry per ray per
 // iteration, so finished lanes are refilled instead of idling.
-template <int STACK, int PER>
+template <int STACK, int PER, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_closest(DevScene s, RayQ q, uint32_t *counters, uint32_t cur,
                                                        uint32_t *hit_ref, float *hit_t,
-                                                       unsigned long long *stats, bool prof) {
+                                                       unsigned long long *stats) {
   const uint32_t n = counters[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     counters[cur ^ 1u] = 0;   // next queue and shadow queue start empty
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_clo
     stats[0] += n;
   }
   TraceCounters c{0, 0, 0};
-  trace_loop<STACK, kClosestOnly, PER>(
+  trace_loop<STACK, kClosestOnly, PER, COUNT>(
       counters + 4, n, c,
       [&](uint32_t ray, Traversal<STACK> &tr, bool &any) {
         const float4 o = q.o[ray], d = q.d[ray];
@@ -134,21 +135,21 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_clo
         hit_t[ray] = tr.t1;
       });
   if (c.overflow) atomicOr(counters + 3, 1u);
-  if (prof) warp_count(stats + 2, c.nodes, c.tests);
+  if (COUNT) warp_count(stats + 2, c.nodes, c.tests);
 }
 
 // Persistent any-hit kernel for the shadow queue (dispenser counters[5]);
 // an unoccluded ray adds its contribution to its path's radiance.
-template <int STACK>
+template <int STACK, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_shadow(DevScene s, ShadowQ q, uint32_t *counters, float4 *rad,
-                                                      unsigned long long *stats, bool prof) {
+                                                      unsigned long long *stats) {
   const uint32_t n = counters[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     stats[1] += n;
     stats[6] += counters[6];   // vertices lit this bounce (DirectIllum::sample_all_lights calls)
   }
   TraceCounters c{0, 0, 0};
-  trace_loop<STACK, kAnyOnly>(
+  trace_loop<STACK, kAnyOnly, 1, COUNT>(
       counters + 5, n, c,
       [&](uint32_t ray, Traversal<STACK> &tr, bool &any) {
         const float4 o = q.o[ray], d = q.d[ray];
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_sha
         atomicAdd(&r->z, cc.z);
       });
   if (c.overflow) atomicOr(counters + 3, 1u);
-  if (prof) warp_count(stats + 4, c.nodes, c.tests);
+  if (COUNT) warp_count(stats + 4, c.nodes, c.tests);
 }
 
 // 6 blocks of 128 per SM (80 registers), as the engine's shading kernels.
@@ -550,27 +551,24 @@ __global__ void __launch_bounds__(256) k_resolve(uint32_t npix, const float4 *ac
   }
 }
 
-template <int STACK>
+template <int STACK, bool COUNT>
 void launch_bounce(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, uint64_t base, uint32_t b,
-                   uint32_t cur, uint32_t grid128, cudaStream_t st, RenderProfile *prof, bool count) {
+                   uint32_t cur, uint32_t grid128, cudaStream_t st, RenderProfile *prof) {
   RayQ qin{wb.q_o[cur], wb.q_d[cur], wb.q_path[cur]};
   RayQ qout{wb.q_o[cur ^ 1], wb.q_d[cur ^ 1], wb.q_path[cur ^ 1]};
   ShadowQ sq{wb.s_o, wb.s_d, wb.s_c};
   DirectL dl{wb.d_idx, wb.d_thr};
   PathPtrs P{wb.thr, wb.rad, wb.pstate, wb.jit};
-  const bool pf = prof != nullptr || count;
+  const auto closest = s.pair_lists ? k_trace_closest<STACK, 2, COUNT> : k_trace_closest<STACK, 1, COUNT>;
+  const auto shadow = k_trace_shadow<STACK, COUNT>;
   if (prof) prof->begin(st, RenderProfile::CLOSEST);
-  if (s.pair_lists)
-    k_trace_closest<STACK, 2><<<resident_grid(k_trace_closest<STACK, 2>, kTraceBlock), kTraceBlock, 0, st>>>(
-        s, qin, wb.counters, cur, wb.hit_ref, wb.hit_t, wb.stats, pf);
-  else
-    k_trace_closest<STACK, 1><<<resident_grid(k_trace_closest<STACK, 1>, kTraceBlock), kTraceBlock, 0, st>>>(
-        s, qin, wb.counters, cur, wb.hit_ref, wb.hit_t, wb.stats, pf);
+  closest<<<resident_grid(closest, kTraceBlock), kTraceBlock, 0, st>>>(s, qin, wb.counters, cur, wb.hit_ref,
+                                                                       wb.hit_t, wb.stats);
   if (prof) prof->end(st), prof->begin(st, RenderProfile::SHADE);
   k_shade<<<grid128, 128, 0, st>>>(s, jc, base, b, qin, wb.counters, cur, wb.hit_ref, wb.hit_t, P, qout, dl);
   k_direct<<<grid128, 128, 0, st>>>(s, jc, base, b, qin, wb.counters, wb.hit_ref, wb.hit_t, dl, sq);
   if (prof) prof->end(st), prof->begin(st, RenderProfile::SHADOW);
-  k_trace_shadow<STACK><<<resident_grid(k_trace_shadow<STACK>, kTraceBlock), kTraceBlock, 0, st>>>(s, sq, wb.counters, wb.rad, wb.stats, pf);
+  shadow<<<resident_grid(shadow, kTraceBlock), kTraceBlock, 0, st>>>(s, sq, wb.counters, wb.rad, wb.stats);
   if (prof) prof->end(st);
 }
 
@@ -770,11 +768,15 @@ cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, 
     nl++;
     for (uint32_t b = 0; b <= jc.max_len; b++) {
       const uint32_t cur = b & 1u;
+      auto bounce = [&](auto stack) {
+        if (prof || count) launch_bounce<stack(), true>(s, jc, wb, base, b, cur, grid128, st, prof);
+        else launch_bounce<stack(), false>(s, jc, wb, base, b, cur, grid128, st, prof);
+      };
       switch (sc) {
-        case 32: launch_bounce<32>(s, jc, wb, base, b, cur, grid128, st, prof, count); break;
-        case 64: launch_bounce<64>(s, jc, wb, base, b, cur, grid128, st, prof, count); break;
-        case 128: launch_bounce<128>(s, jc, wb, base, b, cur, grid128, st, prof, count); break;
-        case 256: launch_bounce<256>(s, jc, wb, base, b, cur, grid128, st, prof, count); break;
+        case 32: bounce(std::integral_constant<int, 32>{}); break;
+        case 64: bounce(std::integral_constant<int, 64>{}); break;
+        case 128: bounce(std::integral_constant<int, 128>{}); break;
+        case 256: bounce(std::integral_constant<int, 256>{}); break;
         default: return cudaErrorInvalidValue;
       }
       nl += 4;
