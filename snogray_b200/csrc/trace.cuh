@@ -191,15 +191,15 @@ __device__ __forceinline__ bool test_prim(const PrimRec &r, float3 o, float3 d, 
 }
 
 // The pending children of one visited node, as one stack record: the
-// node's near-half lower bounds, midpoints and far-half upper bounds (every
-// child's slab bounds are a selection of these, per axis), its first child's
-// index, its child mask and the children not yet entered (by octant bits).  One record per visited node with two or more qualifying children,
+// node's lower bounds and half extents along the ray (a child's bounds are lo
+// or mid = lo + half, and its lower bound + half, per axis), its first child's
+// index, its child mask and the children not yet entered (by octant bits).
+// One record per visited node with two or more qualifying children,
 // instead of one entry per waiting child: a visit pushes at most once, and
 // the stack holds at most one record per tree level.
 struct StackRec {
-  float4 a;   // near_lo.xyz, first child index
-  float4 b;   // mid.xyz, child mask | children still to enter << 8
-  float4 c;   // far.xyz
+  float4 a;   // lo.xyz, first child index
+  float4 b;   // half.xyz, child mask | children still to enter << 8
 };
 
 // Threads per block of every trace kernel.
@@ -213,17 +213,17 @@ constexpr int kTraceBlock = 128;
 // a ring; older ones spill to the thread's local-memory array.  Lanes of a
 // warp sit at different stack depths, so a local-memory stack is read and
 // written uncoalesced; the ring keeps the pushes and pops of a walk on chip
-// (kRing * 48 bytes per thread, 18 KB per 128-thread block at kRing = 3).
+// (kRing * 32 bytes per thread, 16 KB per 128-thread block at kRing = 4).
 #ifndef SNOG_RING
-#define SNOG_RING 3
+#define SNOG_RING 4
 #endif
 constexpr uint32_t kRing = SNOG_RING;
 
-// This thread's first ring slot.  Part k (0, 1, 2) of record position e of
-// thread t is float4 (3 * e + k) * kTraceBlock + t: a warp touching one part
+// This thread's first ring slot.  Part k (0, 1) of record position e of
+// thread t is float4 (2 * e + k) * kTraceBlock + t: a warp touching one part
 // of one position reads 512 contiguous bytes.
 __device__ __forceinline__ float4 *ring_slots() {
-  __shared__ float4 ring[3 * kRing * kTraceBlock];
+  __shared__ float4 ring[2 * kRing * kTraceBlock];
   return ring + threadIdx.x;
 }
 
@@ -237,9 +237,10 @@ __device__ __forceinline__ uint4 *ray_slots() {
   return rays;
 }
 
-constexpr uint32_t kGateFlag = 8u;   // entry carries a parent gate
 constexpr uint32_t kSlowSlab = 8u;   // in Traversal::octant: slab bounds may be NaN
 constexpr uint32_t kAnyHit = 16u;    // in Traversal::octant: an any-hit query
+constexpr uint32_t kGateFlag = 32u;  // in Traversal::octant: the entry carries a parent gate,
+constexpr uint32_t kGateShift = 6u;  //   whose octant bits start here
 enum { kClosestOnly = 0, kAnyOnly = 1, kMixed = 2 };   // queries a trace kernel runs
 
 __device__ __forceinline__ bool slab_open(float t0, float t1, float3 lo, float3 hi) {
@@ -275,11 +276,11 @@ __device__ __forceinline__ uint32_t first_child(uint32_t vm) {
 }
 
 // A resumable octree walk for one ray.  init() sets up the root's slab
-// bounds (space/octree.cc:119-135); node_step() processes one octree entry --
-// the child entered last, else the top of the stack -- as one call of the
-// reference's recursive function does: parent gate, slab cull, then the
-// node's surface list (left pending in [lp, lend) for list_round) and the
-// children.  Kernels interleave the steps of many rays per warp and refill
+// bounds (space/octree.cc:119-135); node_step() processes the current octree
+// entry as one call of the reference's recursive function does: parent gate,
+// slab cull, then the node's surface list (left pending in [lp, lend) for
+// list_round) and the children, the first of which -- or else the next child
+// waiting on the stack -- becomes the current entry.  Kernels interleave the steps of many rays per warp and refill
 // lanes whose ray has finished.  The stack holds one record per tree level
 // on the walk's path; kRecs (from STACK, which the host picks from the tree
 // depth) plus kRing records cover every tree the host admits.  Should they
@@ -288,11 +289,12 @@ template <int STACK>
 struct Traversal {
   float3 lo, hi;
   float t0, t1;
-  uint32_t node, gate, octant, hit_ref;   // octant: bits 0-2, kSlowSlab, kAnyHit
-  uint32_t lp, lend;         // surface list still to test: plist[lp, lend)
-  uint32_t ring;             // shared-memory ring: oldest position | count << 4 (0 when empty)
-  int sp;                    // entries spilled to stk[0, sp)
-  bool have;                 // a current entry (node/gate/lo/hi) is set
+  uint32_t node, octant, hit_ref;   // octant: the ray's in bits 0-2, kSlowSlab, kAnyHit, the entry's gate
+  uint32_t lp, lend;         // surface list still to test: plist[lp, lend), lp <= lend
+  uint32_t ring;             // shared-memory ring: position of its newest record
+  uint32_t held;             // records in the ring
+  int sp;                    // older records, in stk[0, sp)
+  bool have;                 // a current entry (node, gate, lo, hi) is set
   const uint4 *nodes;        // the ray's scene (its list and primitive arrays are in the ray slot)
   // Records the stack may need: one per tree level.  STACK, the class the
   // host picks from the tree depth (at least 3 * depth + 4), bounds them
@@ -324,8 +326,8 @@ struct Traversal {
     hit_ref = PREF_END;
     sp = 0;
     ring = 0;
+    held = 0;
     node = 0;
-    gate = 0;
     lp = lend = 0;
     have = s.n_nodes != 0;
     nodes = s.nodes;
@@ -365,73 +367,30 @@ struct Traversal {
     if (!finite) octant |= kSlowSlab;
   }
 
-  // The walk is over: no list pending, no current entry, empty stack.
-  __device__ __forceinline__ bool finished() const { return lp >= lend && !have && sp == 0 && (ring >> 4) == 0u; }
+  // The walk is over: no list pending, no current entry.
+  __device__ __forceinline__ bool finished() const { return lp == lend && !have; }
 
-  // Push a record: into the ring, first moving the ring's oldest record to
-  // local memory when the ring is full.
-  __device__ __forceinline__ void push(float3 nlo, float3 mid, float3 far, uint32_t first, uint32_t bits,
-                                       TraceCounters &cnt) {
-    float4 *r = ring_slots();
-    uint32_t base = ring & 15u, n = ring >> 4;
-    if (n == kRing) {
+  // Push a record: into the ring, first moving the ring's oldest record --
+  // the one after the newest -- to local memory when the ring is full.
+  __device__ __forceinline__ void push(float3 half, uint32_t first, uint32_t bits, TraceCounters &cnt) {
+    ring = (ring + 1u) % kRing;
+    float4 *r = ring_slots() + 2u * kTraceBlock * ring;
+    if (held == kRing) {
       if (sp < kRecs) {
-        stk[sp].a = r[(3 * base) * kTraceBlock];
-        stk[sp].b = r[(3 * base + 1) * kTraceBlock];
-        stk[sp].c = r[(3 * base + 2) * kTraceBlock];
+        stk[sp].a = r[0];
+        stk[sp].b = r[kTraceBlock];
         sp++;
       } else {
         cnt.overflow = 1;
       }
-      base = base + 1u == kRing ? 0u : base + 1u;
-      n--;
-    }
-    uint32_t pos = base + n;
-    pos = pos >= kRing ? pos - kRing : pos;
-    r[(3 * pos) * kTraceBlock] = make_float4(nlo.x, nlo.y, nlo.z, __uint_as_float(first));
-    r[(3 * pos + 1) * kTraceBlock] = make_float4(mid.x, mid.y, mid.z, __uint_as_float(bits));
-    r[(3 * pos + 2) * kTraceBlock] = make_float4(far.x, far.y, far.z, 0.f);
-    ring = base | ((n + 1u) << 4);
-  }
-
-  // Make the next waiting child of the newest record the current entry (the
-  // record is dropped once its last child is taken).  Returns false, leaving
-  // the walk unchanged, if nothing is stacked.
-  __device__ __forceinline__ bool pop() {
-    float4 *r = ring_slots();
-    uint32_t base = ring & 15u, n = ring >> 4;
-    if (n == 0u) {
-      if (sp == 0) return false;
-      --sp;   // bring the newest spilled record back into the ring
-      r[0] = stk[sp].a;
-      r[kTraceBlock] = stk[sp].b;
-      r[2 * kTraceBlock] = stk[sp].c;
-      base = 0u;
-      n = 1u;
-    }
-    uint32_t pos = base + n - 1u;
-    pos = pos >= kRing ? pos - kRing : pos;
-    const float4 ra = r[(3 * pos) * kTraceBlock], rb = r[(3 * pos + 1) * kTraceBlock],
-                 rc = r[(3 * pos + 2) * kTraceBlock];
-    const uint32_t bits = __float_as_uint(rb.w);
-    const uint32_t vm = bits >> 8;
-    const uint32_t cb = first_child(vm);
-    const uint32_t rest = vm & ~(1u << cb);
-    if (rest) {
-      reinterpret_cast<uint32_t *>(r + (3 * pos + 1) * kTraceBlock)[3] = (bits & 0xffu) | (rest << 8);
-      ring = base | (n << 4);
     } else {
-      ring = n > 1u ? (base | ((n - 1u) << 4)) : 0u;   // an emptied ring restarts at position 0
+      held++;
     }
-    const uint32_t slot = cb ^ (octant & 7u);
-    node = __float_as_uint(ra.w) + __popc(bits & 0xffu & ((1u << slot) - 1u));
-    gate = cb | kGateFlag;
-    lo = f3((cb & 4) ? rb.x : ra.x, (cb & 2) ? rb.y : ra.y, (cb & 1) ? rb.z : ra.z);
-    hi = f3((cb & 4) ? rc.x : rb.x, (cb & 2) ? rc.y : rb.y, (cb & 1) ? rc.z : rb.z);
-    return true;
+    r[0] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(first));
+    r[kTraceBlock] = make_float4(half.x, half.y, half.z, __uint_as_float(bits));
   }
 
-  // One octree entry (call only with no list pending and !finished()).
+  // One octree entry (call only with a current entry and no list pending).
   //
   // An entry is processed as one call of the reference's recursive function:
   // parent gate, slab cull, then the node's surface list, then its children.
@@ -445,12 +404,10 @@ struct Traversal {
   // COUNT: node calls are counted.
   template <int ANY, bool COUNT>
   __device__ __forceinline__ void node_step(TraceCounters &cnt) {
-    if (!have && !pop()) return;
-    have = false;
     const bool slow = octant & kSlowSlab;
     bool open = true;
     const bool any_query = ANY == kAnyOnly || (ANY == kMixed && (octant & kAnyHit));
-    if ((gate & kGateFlag) && any_query) {
+    if ((octant & kGateFlag) && any_query) {
       // An any-hit query's extent never changes, so an entry with a parent
       // gate passed the very gate and cull it would be given now when it
       // was pushed (or entered): the call happens and the node is open.
@@ -458,84 +415,126 @@ struct Traversal {
     } else {
       // The cull decides alone where bounds are finite: it closes whatever the
       // gate does.  The gate is where a call is counted.
-      if ((COUNT || slow) && (gate & kGateFlag)) open = gate_open(gate & 7u, t0, t1, lo, hi);
+      if ((COUNT || slow) && (octant & kGateFlag)) open = gate_open(octant >> kGateShift, t0, t1, lo, hi);
       if (open) {
         if (COUNT) cnt.nodes++;
         open = slow ? slab_open(t0, t1, lo, hi) : slab_open_finite(t0, t1, lo, hi);
       }
-      if (!open) return;
     }
-    const uint4 nd = __ldg(nodes + node);
-    lp = nd.z;
-    lend = nd.z + nd.w;
-    if (!nd.y) return;
-    // (hi - lo) / 2: halving rounds exactly like the reference's division by 2.
-    const float3 half = f3(__fmul_rn(__fsub_rn(hi.x, lo.x), 0.5f), __fmul_rn(__fsub_rn(hi.y, lo.y), 0.5f),
-                           __fmul_rn(__fsub_rn(hi.z, lo.z), 0.5f));
-    // Per axis the children's bounds take two values each: the near half
-    // spans [lo, lo + half], the far half [lo + half, lo + half + half] --
-    // the same rounded sums as the reference's child ranges.
-    const float3 mid = f3(__fadd_rn(lo.x, half.x), __fadd_rn(lo.y, half.y), __fadd_rn(lo.z, half.z));
-    const float3 far = f3(__fadd_rn(mid.x, half.x), __fadd_rn(mid.y, half.y), __fadd_rn(mid.z, half.z));
-    // Which children pass gate and cull, by octant bits.  At most 4 pass: one
-    // octant per crossing of each of the three midplanes.
-    const uint32_t oct = octant & 7u;
-    uint32_t vm = 0;
-    if (slow) {
+    // The record whose children come next: the node's own if any of them
+    // qualifies, else the newest on the stack.
+    float3 half = lo;
+    uint32_t first = 0, bits = 0, vm = 0;   // bits: child mask, children of a stacked record still to enter << 8
+    if (open) {
+      const uint4 nd = __ldg(nodes + node);
+      lp = nd.z;
+      lend = nd.z + nd.w;
+      first = nd.x;
+      bits = nd.y & 0xffu;
+      if (nd.y) {
+        // (hi - lo) / 2: halving rounds exactly like the reference's division by 2.
+        half = f3(__fmul_rn(__fsub_rn(hi.x, lo.x), 0.5f), __fmul_rn(__fsub_rn(hi.y, lo.y), 0.5f),
+                  __fmul_rn(__fsub_rn(hi.z, lo.z), 0.5f));
+        // Per axis the children's bounds take two values each: the near half
+        // spans [lo, lo + half], the far half [lo + half, lo + half + half] --
+        // the same rounded sums as the reference's child ranges.
+        const float3 mid = f3(__fadd_rn(lo.x, half.x), __fadd_rn(lo.y, half.y), __fadd_rn(lo.z, half.z));
+        const float3 far = f3(__fadd_rn(mid.x, half.x), __fadd_rn(mid.y, half.y), __fadd_rn(mid.z, half.z));
+        // Which children pass gate and cull, by octant bits.  At most 4 pass: one
+        // octant per crossing of each of the three midplanes.
+        const uint32_t oct = octant & 7u;
+        if (slow) {
 #pragma unroll
-      for (uint32_t cb = 0; cb < 8; cb++) {
-        const float3 clo = f3((cb & 4) ? mid.x : lo.x, (cb & 2) ? mid.y : lo.y, (cb & 1) ? mid.z : lo.z);
-        const float3 chi = f3((cb & 4) ? far.x : mid.x, (cb & 2) ? far.y : mid.y, (cb & 1) ? far.z : mid.z);
-        const bool ok = ((nd.y >> (cb ^ oct)) & 1u) & gate_open(cb, t0, t1, clo, chi) & slab_open(t0, t1, clo, chi);
-        vm |= ok ? (1u << cb) : 0u;
+          for (uint32_t cb = 0; cb < 8; cb++) {
+            const float3 clo = f3((cb & 4) ? mid.x : lo.x, (cb & 2) ? mid.y : lo.y, (cb & 1) ? mid.z : lo.z);
+            const float3 chi = f3((cb & 4) ? far.x : mid.x, (cb & 2) ? far.y : mid.y, (cb & 1) ? far.z : mid.z);
+            const bool ok =
+                ((nd.y >> (cb ^ oct)) & 1u) & gate_open(cb, t0, t1, clo, chi) & slab_open(t0, t1, clo, chi);
+            vm |= ok ? (1u << cb) : 0u;
+          }
+        } else {
+          // The same tests taken apart.  lo <= mid <= far per axis (half is not
+          // negative where the node is open), so a child's entry is the largest
+          // of ENTRY and the midpoints of its far axes, its exit the smallest of
+          // EXIT and the midpoints of its near axes, and entry < exit holds
+          // exactly when each of the former is below each of the latter: a far
+          // axis' midpoint below EXIT, a near one's above ENTRY, and a far axis'
+          // midpoint below a near one's.  Each failed comparison takes its
+          // children out of the mask.  The gates follow from the same
+          // comparisons.  (Against a maximum, a minimum and four gates for each of
+          // eight children: terrain frame 224.5 -> 201.8 ms, 16M rays in 1M
+          // triangles 20.2 -> 17.6 ms, with the uncounted cull above.)
+          const float entry = fmaxf(fmaxf(t0, lo.x), fmaxf(lo.y, lo.z));
+          const float exit = fminf(fminf(t1, far.x), fminf(far.y, far.z));
+          vm = (__byte_perm(nd.y, 0u, (oct & 3u) * 0x1111u) >> (oct & 4u)) & 0xffu;   // children that exist
+          if (!(entry < exit)) vm = 0u;
+          if (!(entry < mid.x)) vm &= 0xf0u;
+          if (!(entry < mid.y)) vm &= 0xccu;
+          if (!(entry < mid.z)) vm &= 0xaau;
+          if (!(mid.x < exit)) vm &= 0x0fu;
+          if (!(mid.y < exit)) vm &= 0x33u;
+          if (!(mid.z < exit)) vm &= 0x55u;
+          if (!(mid.x < mid.y)) vm &= ~0x30u;   // x far, y near
+          if (!(mid.y < mid.x)) vm &= ~0x0cu;
+          if (!(mid.x < mid.z)) vm &= ~0x50u;   // x far, z near
+          if (!(mid.z < mid.x)) vm &= ~0x0au;
+          if (!(mid.y < mid.z)) vm &= ~0x44u;   // y far, z near
+          if (!(mid.z < mid.y)) vm &= ~0x22u;
+        }
       }
-    } else {
-      // The same tests taken apart.  lo <= mid <= far per axis (half is not
-      // negative where the node is open), so a child's entry is the largest
-      // of ENTRY and the midpoints of its far axes, its exit the smallest of
-      // EXIT and the midpoints of its near axes, and entry < exit holds
-      // exactly when each of the former is below each of the latter: a far
-      // axis' midpoint below EXIT, a near one's above ENTRY, and a far axis'
-      // midpoint below a near one's.  Each failed comparison takes its
-      // children out of the mask.  The gates follow from the same
-      // comparisons.  (Against a maximum, a minimum and four gates for each of
-      // eight children: terrain frame 224.5 -> 201.8 ms, 16M rays in 1M
-      // triangles 20.2 -> 17.6 ms, with the uncounted cull above.)
-      const float entry = fmaxf(fmaxf(t0, lo.x), fmaxf(lo.y, lo.z));
-      const float exit = fminf(fminf(t1, far.x), fminf(far.y, far.z));
-      vm = (__byte_perm(nd.y, 0u, (oct & 3u) * 0x1111u) >> (oct & 4u)) & 0xffu;   // children that exist
-      if (!(entry < exit)) vm = 0u;
-      if (!(entry < mid.x)) vm &= 0xf0u;
-      if (!(entry < mid.y)) vm &= 0xccu;
-      if (!(entry < mid.z)) vm &= 0xaau;
-      if (!(mid.x < exit)) vm &= 0x0fu;
-      if (!(mid.y < exit)) vm &= 0x33u;
-      if (!(mid.z < exit)) vm &= 0x55u;
-      if (!(mid.x < mid.y)) vm &= ~0x30u;   // x far, y near
-      if (!(mid.y < mid.x)) vm &= ~0x0cu;
-      if (!(mid.x < mid.z)) vm &= ~0x50u;   // x far, z near
-      if (!(mid.z < mid.x)) vm &= ~0x0au;
-      if (!(mid.y < mid.z)) vm &= ~0x44u;   // y far, z near
-      if (!(mid.z < mid.y)) vm &= ~0x22u;
     }
-    if (!vm) return;
     // The first qualifying child becomes the current entry; the others wait
     // in one record and are entered in visiting order after the first
-    // child's subtree (pop), as the reference's loop over the children does.
+    // child's subtree, as the reference's loop over the children does.
+    const bool popped = vm == 0u;
+    if (popped) {
+      float4 ra, rb;
+      if (held) {
+        const float4 *r = ring_slots() + 2u * kTraceBlock * ring;
+        ra = r[0];
+        rb = r[kTraceBlock];
+      } else if (sp) {
+        ra = stk[sp - 1].a;
+        rb = stk[sp - 1].b;
+      } else {
+        have = false;
+        return;
+      }
+      lo = xyz(ra);
+      half = xyz(rb);
+      first = __float_as_uint(ra.w);
+      bits = __float_as_uint(rb.w);
+      vm = bits >> 8;
+    }
     const uint32_t cb = first_child(vm);
     const uint32_t rest = vm & ~(1u << cb);
-    if (rest) push(lo, mid, far, nd.x, (nd.y & 0xffu) | (rest << 8), cnt);
-    const uint32_t slot = cb ^ oct;
-    node = nd.x + __popc(nd.y & ((1u << slot) - 1u));
-    gate = cb | kGateFlag;
-    lo = f3((cb & 4) ? mid.x : lo.x, (cb & 2) ? mid.y : lo.y, (cb & 1) ? mid.z : lo.z);
-    hi = f3((cb & 4) ? far.x : mid.x, (cb & 2) ? far.y : mid.y, (cb & 1) ? far.z : mid.z);
-    have = true;
+    const uint32_t word = (bits & 0xffu) | (rest << 8);
+    if (!popped) {
+      if (rest) push(half, first, word, cnt);
+    } else if (held) {
+      if (rest) {
+        reinterpret_cast<uint32_t *>(ring_slots() + (2u * ring + 1u) * kTraceBlock)[3] = word;
+      } else {
+        held--;
+        ring = (ring + kRing - 1u) % kRing;
+      }
+    } else if (rest) {
+      stk[sp - 1].b.w = __uint_as_float(word);
+    } else {
+      sp--;
+    }
+    node = first + __popc(bits & ((1u << (cb ^ (octant & 7u))) - 1u));
+    octant = (octant & (kGateFlag - 1u)) | kGateFlag | (cb << kGateShift);
+    // The far half starts at mid; either half ends half an extent after it starts.
+    if (cb & 4) lo.x = __fadd_rn(lo.x, half.x);
+    if (cb & 2) lo.y = __fadd_rn(lo.y, half.y);
+    if (cb & 1) lo.z = __fadd_rn(lo.z, half.z);
+    hi = f3(__fadd_rn(lo.x, half.x), __fadd_rn(lo.y, half.y), __fadd_rn(lo.z, half.z));
   }
 };
 
 // One warp-cooperative round of list tests.  Every lane with a list pending
-// (WANT) owns the next entries of its list; the warp's pending entries, in
+// owns the next entries of its list; the warp's pending entries, in
 // lane order and list order, are dealt to its 32 lanes (one or two
 // consecutive entries per lane: at most 32 or 64 per round), each lane tests
 // its entries against its owner's ray, and each owner takes the result of its
@@ -566,11 +565,11 @@ struct Traversal {
 // and a five-shuffle search per unit: terrain frame 273.3 -> 225.5 ms, 16M
 // rays in 1M triangles 24.7 -> 20.15 ms.)
 template <int STACK, int ANY, int PER>
-__device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool any, TraceCounters &cnt) {
+__device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool any, TraceCounters &cnt) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr uint32_t kPer = uint32_t(PER);
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t c = want ? tr.lend - tr.lp : 0u;
+  uint32_t c = tr.lend - tr.lp;
   c = c < 32u * kPer ? c : 32u * kPer;
   const uint32_t np = (c + kPer - 1u) / kPer;   // dealt units: pairs (or entries)
   uint32_t incl = np;
@@ -668,20 +667,28 @@ __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool want, bool
   return over;
 }
 
-// Idle lanes a warp gathers before it refills them (1 = refill at once).
+// Idle lanes a warp gathers before it refills them (1 = refill at once): 8 in
+// the renderers' kernels, 4 in the ray-batch kernel, whose ray starts read
+// less (terrain frame 193.0 ms at 4, 190.9 at 8; 1M rays among 22k mixed
+// primitives 0.82 ms at 4, 0.86 at 8).
 #ifndef SNOG_REFILL_MIN
-#define SNOG_REFILL_MIN 4
+#define SNOG_REFILL_MIN 8
 #endif
-constexpr uint32_t kRefillMin = SNOG_REFILL_MIN;
+constexpr uint32_t refill_min(int any) { return any == kMixed ? 4u : uint32_t(SNOG_REFILL_MIN); }
 
-// Pending list entries a closest-hit warp gathers before a list round.
+// Pending list entries a closest-hit warp gathers before a list round, and
+// the lanes able to visit a node below which it does not wait for more
+// (closest-hit kernel of the terrain frame 77.2 ms at 24 and 0, 76.3 at 16
+// and 4).
 #ifndef SNOG_ROUND_MIN
-#define SNOG_ROUND_MIN 24
+#define SNOG_ROUND_MIN 16
 #endif
 constexpr uint32_t kRoundMin = SNOG_ROUND_MIN;
+constexpr uint32_t kFewSteps = 4;
 // A warp with fewer than 32 entries pending visits nodes, and one with at
-// least kRoundMin runs a round; a threshold above 32 would leave a warp with
-// 32..kRoundMin-1 entries pending doing neither, for ever.
+// least kRoundMin, or no lane that could visit one, runs a round; a threshold
+// above 32 would leave a warp with 32..kRoundMin-1 entries pending doing
+// neither, for ever.
 static_assert(kRoundMin >= 1u && kRoundMin <= 32u, "closest-hit round threshold must not exceed the node-step cut");
 
 // Warp-cooperative ray dispenser for the persistent trace kernels: lanes
@@ -700,8 +707,7 @@ static_assert(kRoundMin >= 1u && kRoundMin <= 32u, "closest-hit round threshold 
 struct RayDispenser {
   static constexpr uint32_t kIdle = 0xffffffffu;
   uint32_t next = 0, end = 0;
-  uint32_t limit;
-  bool exhausted = false;
+  uint32_t limit;   // 0: no rays remain to be handed out
 
   __device__ __forceinline__ explicit RayDispenser(uint32_t n) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -709,32 +715,25 @@ struct RayDispenser {
     limit = share < 1u ? 1u : share < 32u ? share : 32u;
   }
 
-  // Returns the new ray index for a lane that asked (NEED) and got one,
-  // else kIdle.  Sets *all_idle when every lane is idle and no rays remain.
-  __device__ __forceinline__ uint32_t fetch(uint32_t *counter, uint32_t n, bool need, bool busy,
-                                            bool *all_idle) {
+  // The new ray index for a lane that asked (NEED) and got one, else kIdle.
+  __device__ __forceinline__ uint32_t fetch(uint32_t *counter, uint32_t n, bool need) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t mask = __ballot_sync(0xffffffffu, need);
-    uint32_t got = kIdle;
-    if (mask) {
-      if (next >= end && !exhausted) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(counter, limit);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) {
-          exhausted = true;
-        } else {
-          next = base;
-          end = base + limit < n ? base + limit : n;
-        }
+    if (next == end) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(counter, limit);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= n) {
+        limit = 0;
+      } else {
+        next = base;
+        end = n - base < limit ? n : base + limit;
       }
-      const uint32_t rank = __popc(mask & ((1u << lane) - 1u));
-      if (need && next + rank < end) got = next + rank;
-      const uint32_t take = __popc(mask);
-      next = (next + take < end) ? next + take : end;
     }
-    const bool idle = !busy && got == kIdle;
-    *all_idle = __all_sync(0xffffffffu, idle) && exhausted && next >= end;
+    const uint32_t rank = __popc(mask & ((1u << lane) - 1u));
+    const uint32_t got = need && rank < end - next ? next + rank : kIdle;
+    const uint32_t take = __popc(mask);
+    next = take < end - next ? next + take : end;
     return got;
   }
 };
@@ -746,6 +745,15 @@ struct RayDispenser {
 // round of list entries pending, every live lane without a list pending
 // visits one octree entry; then the warp tests one round of pending list
 // entries together.  All 32 lanes of every warp must run it.
+//
+// The loop is bound by instructions issued: on the terrain frame the
+// closest-hit kernel runs 0.86 node steps (25.8 lanes on average), 0.76 list
+// rounds (31.1 entries) and 0.24 refills an iteration, so what counts is
+// the length of each.  Against popping the next entry at the start of a step,
+// a third 16-byte part per stack record and a vote on every refill, with
+// the ring of 4 records that the smaller ones make room for: terrain frame
+// 201.9 -> 190.9 ms, 16M rays in 1M triangles 17.6 -> 16.4 ms, 200k-triangle
+// soup 19.8 -> 17.7 ms.
 template <int STACK, int ANY, int PER, bool COUNT, class Start, class Done>
 __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, TraceCounters &cnt, Start start,
                                            Done done) {
@@ -753,45 +761,45 @@ __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, Trac
   Traversal<STACK> tr;
   tr.stk = stk;
   RayDispenser disp(n);
-  const bool takes = (threadIdx.x & 31u) < disp.limit;
-  const uint32_t refill_min = kRefillMin < disp.limit ? kRefillMin : disp.limit;
+  tr.have = false;
+  tr.lp = tr.lend = 0;
   uint32_t ray = RayDispenser::kIdle;
   bool any = false;
+  // Idle lanes take new rays only once refill_min of those that may are idle:
+  // a ray start (queue loads, root slab set-up, ray slot) then runs on several
+  // lanes at once instead of on one or two every iteration.
   for (;;) {
-    bool all_idle;
-    // Idle lanes take new rays only once kRefillMin of them are idle: a ray
-    // start (queue loads, root slab set-up, ray slot) then runs on several
-    // lanes at once instead of on one or two every iteration.
-    const uint32_t idle_lanes = __popc(__ballot_sync(0xffffffffu, takes && ray == RayDispenser::kIdle));
-    const bool need = takes && ray == RayDispenser::kIdle && idle_lanes >= refill_min;
-    const uint32_t got = disp.fetch(dispenser, n, need, ray != RayDispenser::kIdle, &all_idle);
-    if (all_idle) break;
-    if (got != RayDispenser::kIdle) {
-      ray = got;
-      start(ray, tr, any);
-      if (any) tr.octant |= kAnyHit;
+    const uint32_t idle = __ballot_sync(0xffffffffu, ray == RayDispenser::kIdle);
+    if (disp.limit == 0u) {
+      if (idle == 0xffffffffu) break;
+    } else if (__popc(idle) + disp.limit >= 32u + (refill_min(ANY) < disp.limit ? refill_min(ANY) : disp.limit)) {
+      const uint32_t got =
+          disp.fetch(dispenser, n, ray == RayDispenser::kIdle && (threadIdx.x & 31u) < disp.limit);
+      if (got != RayDispenser::kIdle) {
+        ray = got;
+        start(ray, tr, any);
+        if (any) tr.octant |= kAnyHit;
+      }
     }
-    const bool busy = ray != RayDispenser::kIdle;
     // Visit nodes only while the warp's pending list entries would not fill
     // a round: list rounds run full, node steps run with more lanes at once.
-    const uint32_t pend = (busy && tr.lp < tr.lend) ? tr.lend - tr.lp : 0u;
+    const uint32_t pend = tr.lend - tr.lp;
     const uint32_t pending = __reduce_add_sync(0xffffffffu, pend < 32u ? pend : 32u);
-    if (pending < 32u && busy && tr.lp >= tr.lend && !tr.finished()) tr.template node_step<ANY, COUNT>(cnt);
-    // Closest-hit kernels test lists only once at least kRoundMin entries
-    // are pending, unless no lane could visit a node: fewer, fuller rounds
-    // (2 % off the terrain frame; the any-hit and mixed kernels, whose
-    // lists are longer or whose walks end early, measured no gain or a
-    // loss).
+    if (pending < 32u && tr.have && pend == 0u) tr.template node_step<ANY, COUNT>(cnt);
+    // Closest-hit kernels test lists only once at least kRoundMin entries are
+    // pending or few lanes could visit a node: fewer, fuller rounds.  (Any-hit
+    // and mixed kernels, whose walks end early or whose lists are longer,
+    // measured a loss: shadow rays of the terrain frame 60.5 -> 62.5 ms.)
     bool round = true;
     if (ANY == kClosestOnly) {
-      const uint32_t pend2 = (busy && tr.lp < tr.lend) ? tr.lend - tr.lp : 0u;
+      const uint32_t pend2 = tr.lend - tr.lp;
       const uint32_t pending2 = __reduce_add_sync(0xffffffffu, pend2 < 32u ? pend2 : 32u);
-      const bool can_step = busy && tr.lp >= tr.lend && !tr.finished();
-      round = pending2 >= kRoundMin || __ballot_sync(0xffffffffu, can_step) == 0u;
+      round = pending2 >= kRoundMin || __popc(__ballot_sync(0xffffffffu, tr.have && pend2 == 0u)) <= kFewSteps;
     }
-    const bool stop = round && list_round<STACK, ANY, PER>(tr, busy && tr.lp < tr.lend, any, cnt);
-    if (busy && (stop || tr.finished())) {
+    const bool stop = round && list_round<STACK, ANY, PER>(tr, any, cnt);
+    if (ray != RayDispenser::kIdle && (stop || tr.finished())) {
       done(ray, tr, any);
+      tr.have = false;
       ray = RayDispenser::kIdle;
     }
   }
