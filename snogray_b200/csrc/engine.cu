@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "engine.h"
 #include "launch.h"
@@ -171,21 +172,51 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_shadow(
   if (c.overflow) atomicOr(&ctl->err, 1u);
 }
 
+// Threads per block of the shading kernels: one block of kLongBlock per SM
+// while many paths are to be traced, free-running blocks of 128 otherwise.
+constexpr int kLongBlock = 896;
+constexpr int shade_blocks(int block) { return block == kLongBlock ? 1 : 6; }   // per SM (72 / 80 registers)
+// Paths left to trace from which the long blocks pay: the engine's terrain
+// renders take 11.43 ms (long: 11.22) at 4.3M paths and 39.8 (38.0) at 17M,
+// Cornell ones 2.73 (2.82) at 1.1M and 34.1 (34.1) at 17M.
+constexpr uint64_t kLongPaths = 1u << 21;
+
+// A thread's items of a shading launch over N items are FIRST + k * STRIDE + OFF
+// while FIRST + k * STRIDE < N; whole warps run each pass together, and in
+// long blocks whole blocks do.
+//
+// The shading bodies are long -- more instructions than the caches next to
+// the schedulers hold -- and warps that drift apart each fetch them again:
+// 4-6 of 10 stalled warps waited for instructions.  In a long block a barrier
+// per pass keeps the warps of an SM within reach of one fetch (terrain frame:
+// shading 40.9 ms with 6 free-running blocks of 128 threads per SM; 34.7 in
+// blocks of 256, 33.4 in one of 768, 32.5 in one of 896; more barriers inside
+// the pass measured no gain).  Long blocks are dealt the warps of a launch
+// with less than a pass in turn, so that it is spread over all SMs; other
+// passes take consecutive items, which share scene records (33.7 ms dealt in
+// turn).
+template <int BLOCK>
+struct ShadeItems {
+  uint32_t first, stride, off;
+  __device__ __forceinline__ explicit ShadeItems(uint32_t n) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    stride = gridDim.x * BLOCK;
+    if (BLOCK == kLongBlock) {
+      first = 0;
+      off = n < stride ? (warp * gridDim.x + blockIdx.x) * 32u + lane : blockIdx.x * BLOCK + threadIdx.x;
+    } else {
+      first = blockIdx.x * BLOCK + warp * 32u;
+      off = lane;
+    }
+  }
+};
+
 // Shading, first half: emission, the continuation sample and roulette; the
-// vertices to light go to a list for k_e_direct.  6 blocks of 128 per SM (80
-// registers) for both halves: the bodies are long and divergent, and more
-// resident warps hide their instruction-fetch stalls (4 or 5 blocks for
-// k_e_direct, 8 for k_e_shade measured 0.6-2 % slower on the terrain frame).
+// vertices to light go to a list for k_e_direct.
 // DIRECT: the direct integrator's code is compiled in (launched while a job
 // of that integrator is active; the path integrator's kernel stays smaller).
-#ifndef SNOG_SHADE_MINBLOCKS
-#define SNOG_SHADE_MINBLOCKS 6
-#endif
-#ifndef SNOG_DIRECT_MINBLOCKS
-#define SNOG_DIRECT_MINBLOCKS 6
-#endif
-template <bool DIRECT>
-__global__ void __launch_bounds__(128, SNOG_SHADE_MINBLOCKS) k_e_shade(EngineCtl *ctl, uint32_t cur, const EngineJobDev *jobs,
+template <bool DIRECT, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, shade_blocks(BLOCK)) k_e_shade(EngineCtl *ctl, uint32_t cur, const EngineJobDev *jobs,
                                                  const DevScene *scenes, EQ qin, const uint32_t *hit_ref,
                                                  const float *hit_t, EQ qout, EDL dl,
                                                  unsigned long long *job_done, unsigned long long *job_spawned,
@@ -193,11 +224,11 @@ __global__ void __launch_bounds__(128, SNOG_SHADE_MINBLOCKS) k_e_shade(EngineCtl
   const uint32_t n = ctl->qcount[cur];
   uint32_t *count_out = &ctl->qcount[cur ^ 1u];
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const ShadeItems<BLOCK> items(n);
 
-  for (uint32_t wb = warp * 32; wb < n; wb += nwarps * 32) {
-    const uint32_t i = wb + lane;
+  for (uint32_t pass = items.first; pass < n; pass += items.stride) {
+    if (BLOCK == kLongBlock) __syncthreads();
+    const uint32_t i = pass + items.off;
     const bool active = i < n;
     uint32_t ps = 0, ref = PREF_END, job = 0, scene = 0, bounce = 0;
     unsigned long long g = 0;
@@ -411,18 +442,18 @@ __global__ void __launch_bounds__(128, SNOG_SHADE_MINBLOCKS) k_e_shade(EngineCtl
 // as in k_e_shade, so the same bits), then every light is sampled.  Kept out
 // of k_e_shade so neither kernel's body outgrows the instruction cache, and
 // run over a compacted list so escaped and absorbed paths leave no idle lanes.
-template <bool DIRECT>
-__global__ void __launch_bounds__(128, SNOG_DIRECT_MINBLOCKS) k_e_direct(EngineCtl *ctl, const EngineJobDev *jobs,
+template <bool DIRECT, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, shade_blocks(BLOCK)) k_e_direct(EngineCtl *ctl, const EngineJobDev *jobs,
                                                   const DevScene *scenes, EQ qin, const uint32_t *hit_ref,
                                                   const float *hit_t, EDL dl, ESQ sq) {
   const uint32_t n = ctl->dcount;
   uint32_t *count_sq = &ctl->scount;
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const ShadeItems<BLOCK> items(n);
 
-  for (uint32_t wb = warp * 32; wb < n; wb += nwarps * 32) {
-    const uint32_t k = wb + lane;
+  for (uint32_t pass = items.first; pass < n; pass += items.stride) {
+    if (BLOCK == kLongBlock) __syncthreads();
+    const uint32_t k = pass + items.off;
     const bool alive = k < n;
     uint32_t scene = 0, bounce = 0, pixel = 0, sidx = 0;
     float3 thr = f3(0, 0, 0);
@@ -553,7 +584,7 @@ template <int STACK, int PER>
 void launch_iteration(cudaStream_t st, EngineCtl *ctl, const WorkItem *ring, uint32_t R, uint32_t N,
                       uint32_t cur, const EngineJobDev *jobs, const DevScene *scenes, EQ qc, EQ qn,
                       uint32_t *hit_ref, float *hit_t, EDL dl, ESQ sq, unsigned long long *job_done,
-                      unsigned long long *job_spawned, EQ sp, uint32_t sp_cap, bool direct,
+                      unsigned long long *job_spawned, EQ sp, uint32_t sp_cap, bool direct, bool long_run,
                       const cudaEvent_t *ev) {
   const uint32_t sms = uint32_t(num_sms());
   if (ev) cudaEventRecord(ev[0], st);
@@ -563,15 +594,17 @@ void launch_iteration(cudaStream_t st, EngineCtl *ctl, const WorkItem *ring, uin
   k_e_closest<STACK, PER><<<resident_grid(k_e_closest<STACK, PER>, kTraceBlock), kTraceBlock, 0, st>>>(
       ctl, cur, jobs, scenes, qc, hit_ref, hit_t);
   if (ev) cudaEventRecord(ev[2], st);
-  if (direct) {
-    k_e_shade<true><<<sms * 12, 128, 0, st>>>(ctl, cur, jobs, scenes, qc, hit_ref, hit_t, qn, dl, job_done,
-                                              job_spawned, sp, sp_cap);
-    k_e_direct<true><<<sms * 12, 128, 0, st>>>(ctl, jobs, scenes, qc, hit_ref, hit_t, dl, sq);
-  } else {
-    k_e_shade<false><<<sms * 12, 128, 0, st>>>(ctl, cur, jobs, scenes, qc, hit_ref, hit_t, qn, dl, job_done,
-                                               job_spawned, sp, sp_cap);
-    k_e_direct<false><<<sms * 12, 128, 0, st>>>(ctl, jobs, scenes, qc, hit_ref, hit_t, dl, sq);
-  }
+  auto shading = [&](auto d, auto block) {
+    constexpr int kBlock = block();
+    const uint32_t grid = sms * (kBlock == kLongBlock ? 1u : 12u);
+    k_e_shade<d(), kBlock><<<grid, kBlock, 0, st>>>(ctl, cur, jobs, scenes, qc, hit_ref, hit_t, qn, dl, job_done,
+                                                    job_spawned, sp, sp_cap);
+    k_e_direct<d(), kBlock><<<grid, kBlock, 0, st>>>(ctl, jobs, scenes, qc, hit_ref, hit_t, dl, sq);
+  };
+  const std::integral_constant<int, kLongBlock> long_block;
+  const std::integral_constant<int, 128> short_block;
+  if (direct) long_run ? shading(std::true_type{}, long_block) : shading(std::true_type{}, short_block);
+  else long_run ? shading(std::false_type{}, long_block) : shading(std::false_type{}, short_block);
   if (ev) cudaEventRecord(ev[3], st);
   k_e_shadow<STACK><<<resident_grid(k_e_shadow<STACK>, kTraceBlock), kTraceBlock, 0, st>>>(ctl, scenes, sq);
   if (ev) cudaEventRecord(ev[4], st);
@@ -699,9 +732,7 @@ Engine::Engine(const EngineConfigHost &cfg, cudaStream_t stream) : cfg_(cfg) {
 Engine::~Engine() {
   if (stream_) cudaStreamSynchronize(stream_);
   for (auto &kv : jobs_) release_job(kv.second);
-  for (auto &row : graph_)
-    for (cudaGraphExec_t &gx : row)
-      if (gx) cudaGraphExecDestroy(gx);
+  drop_graphs();
   cache_.trim();
   cudaFree(block_);
   cudaFreeHost(ctl_host_);
@@ -709,6 +740,15 @@ Engine::~Engine() {
   cudaFreeHost(staging_);
   for (cudaEvent_t e : events_) cudaEventDestroy(e);
   if (own_stream_) cudaStreamDestroy(stream_);
+}
+
+void Engine::drop_graphs() {
+  for (auto &by_pair : graph_)
+    for (auto &by_length : by_pair)
+      for (cudaGraphExec_t &gx : by_length) {
+        if (gx) cudaGraphExecDestroy(gx);
+        gx = nullptr;
+      }
 }
 
 void Engine::reset_scenes() {
@@ -741,11 +781,7 @@ uint32_t Engine::add_scene(SceneImpl *scene) {
   check_cuda(cudaStreamSynchronize(stream_), "scene table");
   const int sc = stack_class_for_depth(scene->dev.max_depth);
   if (sc > graph_stack_) {
-    for (auto &row : graph_)
-      for (cudaGraphExec_t &gx : row) {
-        if (gx) cudaGraphExecDestroy(gx);
-        gx = nullptr;
-      }
+    drop_graphs();
     graph_stack_ = sc;
   }
   return slot;
@@ -753,7 +789,7 @@ uint32_t Engine::add_scene(SceneImpl *scene) {
 
 // Every iteration of one launch (iters_per_launch pairs, queue 0 -> 1 -> 0),
 // with events around the kernels while profiling.
-void Engine::launch_iterations(bool direct, bool pair) {
+void Engine::launch_iterations(bool direct, bool pair, bool long_run) {
   EQ q[2];
   for (int k = 0; k < 2; k++) q[k] = EQ{q_o_[k], q_d_[k], q_thr_[k], q_rad_[k], q_meta_[k]};
   ESQ sq{s_o_, s_d_, s_c_, s_tgt_};
@@ -772,7 +808,7 @@ void Engine::launch_iterations(bool direct, bool pair) {
   launch_iteration<S, P>(stream_, ctl_, ring_, cfg_.ring_items, cfg_.slots, cur, jobs_dev_, scenes_dev_, q[cur], \
                          q[cur ^ 1], hit_ref_, hit_t_, EDL{d_idx_, d_tgt_}, sq, job_done_,                      \
                          job_done_ + cfg_.max_jobs, EQ{sp_o_, sp_d_, sp_thr_, sp_rad_, sp_meta_}, sp_cap_,     \
-                         direct, ev)
+                         direct, long_run, ev)
     switch (graph_stack_ * 2 + (pair ? 1 : 0)) {
       case 64: SNOG_ITER(32, 1); break;
       case 65: SNOG_ITER(32, 2); break;
@@ -787,16 +823,16 @@ void Engine::launch_iterations(bool direct, bool pair) {
   }
 }
 
-void Engine::build_graph(bool direct, bool pair) {
+void Engine::build_graph(bool direct, bool pair, bool long_run) {
   cudaGraph_t g;
   const bool prof = profile_on_;
   profile_on_ = false;
   check_cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
-  launch_iterations(direct, pair);
+  launch_iterations(direct, pair, long_run);
   profile_on_ = prof;
   cudaError_t e = cudaStreamEndCapture(stream_, &g);
   check_cuda(e, "end capture");
-  e = cudaGraphInstantiate(&graph_[direct][pair], g, 0);
+  e = cudaGraphInstantiate(&graph_[direct][pair][long_run], g, 0);
   cudaGraphDestroy(g);
   check_cuda(e, "graph instantiate");
 }
@@ -1103,12 +1139,13 @@ bool Engine::step() {
     (scenes_[j.scene_slot]->dev.pair_lists ? paired : single) += left;
   }
   const bool pair = paired > single;
+  const bool long_run = paired + single >= kLongPaths;   // shading in long blocks
   if (work) {
     if (profile_on_) {
-      launch_iterations(direct, pair);
+      launch_iterations(direct, pair, long_run);
     } else {
-      if (!graph_[direct][pair]) build_graph(direct, pair);
-      check_cuda(cudaGraphLaunch(graph_[direct][pair], stream_), "graph launch");
+      if (!graph_[direct][pair][long_run]) build_graph(direct, pair, long_run);
+      check_cuda(cudaGraphLaunch(graph_[direct][pair][long_run], stream_), "graph launch");
     }
     kernel_launches_ += 6 * 2 * cfg_.iters_per_launch;
     check_cuda(cudaMemcpyAsync(ctl_host_, ctl_, sizeof(EngineCtl), cudaMemcpyDeviceToHost, stream_), "ctl");
