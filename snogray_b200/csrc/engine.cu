@@ -448,7 +448,6 @@ __global__ void __launch_bounds__(BLOCK, shade_blocks(BLOCK)) k_e_direct(EngineC
                                                   const float *hit_t, EDL dl, ESQ sq) {
   const uint32_t n = ctl->dcount;
   uint32_t *count_sq = &ctl->scount;
-  const uint32_t lane = threadIdx.x & 31u;
   const ShadeItems<BLOCK> items(n);
 
   for (uint32_t pass = items.first; pass < n; pass += items.stride) {
