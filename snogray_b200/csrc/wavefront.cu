@@ -433,100 +433,167 @@ __global__ void __launch_bounds__(128, 6) k_direct(DevScene s, JobConsts jc, uin
 }
 
 // ImageMitchellFilt::mitchell1 with B = C = 1/3, radius 2
-// (image/image-mitchell-filt.h:50-65).
+// (image/image-mitchell-filt.h:50-65): both cubics by fused Horner steps, which
+// round once where the reference's expression rounds three times, and a select.
 __device__ __forceinline__ float mitchell1(float x) {
-  const float b = 1.f / 3.f, c = 1.f / 3.f;
+  constexpr double b = 1.0 / 3.0, c = 1.0 / 3.0;
   x = fabsf(x);
-  if (x > 2.f) return 0.f;
-  if (x > 1.f)
-    return ((-b - 6 * c) * x * x * x + (6 * b + 30 * c) * x * x + (-12 * b - 48 * c) * x + (8 * b + 24 * c)) *
-           (1.f / 6.f);
-  return ((12 - 9 * b - 6 * c) * x * x * x + (-18 + 12 * b + 6 * c) * x * x + (6 - 2 * b)) * (1.f / 6.f);
+  const float inner = fmaf(fmaf(float((12 - 9 * b - 6 * c) / 6), x, float((-18 + 12 * b + 6 * c) / 6)), x * x,
+                           float((6 - 2 * b) / 6));
+  const float outer = fmaf(fmaf(fmaf(float((-b - 6 * c) / 6), x, float((6 * b + 30 * c) / 6)), x,
+                                float((-12 * b - 48 * c) / 6)),
+                           x, float((8 * b + 24 * c) / 6));
+  return x > 2.f ? 0.f : x > 1.f ? outer : inner;
 }
+
+// Target pixels of a splat block: a thread takes kSplatRows of one column.
+constexpr int kSplatW = 32, kSplatRows = 4, kSplatWarps = 4, kSplatH = kSplatRows * kSplatWarps;
+constexpr int kHaloW = kSplatW + 4, kHaloH = kSplatH + 4, kHalo = kHaloW * kHaloH;
 
 // Gather the wave's samples into the target pixels they reach
 // (ImageFilterConv::add_sample, image/image-filter-conv.h:109-186): every
 // sample within the filter's support of a target pixel centre adds
 // Tint * w and w, with the negative-lobe clamp (neg_clamp = -0.1).
-// G lanes (a power of two up to 32) per target pixel: they take every G-th
-// sample of each neighbouring pattern pixel -- consecutive samples, so the
-// group's loads coalesce -- and sum their shares with shuffles.  With one
-// thread per pixel a small image at high spp left most of the GPU idle on
-// long chains of loads.
-template <int G>
-__global__ void __launch_bounds__(256) k_splat(JobConsts jc, uint64_t base, uint32_t n, const float4 *rad,
-                                               const float2 *jit, float4 *accum, float *wsum, int ty0,
-                                               int nrows) {
+//
+// Every sample reaches 25 pixels, so what a pixel and a sample cost together
+// is what counts.  A block takes one sample of each pattern pixel around its
+// 32x16 targets at a time: first each sample's colour, its five weights per
+// axis and its clamp go to shared memory, then every thread adds the products
+// for its four targets -- two products, five fused additions and no branch
+// each, with a sample's colour read once for up to four targets.  The clamp
+// scales a product whose smallest component lies below -0.1 to it, which is
+// to say that the weight is at least -0.1 / largest component.
+// The blocks of one tile take every gridDim.x-th sample each; with more than
+// one, the sums meet in atomic additions, so small images at many samples fill
+// the device too, and the tile's blocks run together, so that what one of them
+// leaves of a memory sector is still in L2 for the next.
+// (Bound by shared-memory latency at 20 warps per SM.  Against lanes that each
+// evaluated the filter for every pair of sample and target: 853x479 pixels at 9
+// samples 817 -> 145 us, 256x256 at 16 136 -> 53 us, at 64 510 -> 176 us.  Two
+// or one target per thread in more warps: 253 and 184 us on the first.)
+template <bool ATOMIC>
+__global__ void __launch_bounds__(32 * kSplatWarps, 5) k_splat(JobConsts jc, uint64_t base, uint32_t n,
+                                                          const float4 *__restrict__ rad,
+                                                          const float2 *__restrict__ jit, float4 *accum, float *wsum,
+                                                          int ty0, int nrows) {
+  __shared__ float4 col[kHalo];                  // alpha-scaled colour, alpha
+  __shared__ float wlo[kHalo];                   // the least weight the clamp lets pass
+  __shared__ float wx[5][kHalo], wy[5][kHalo];   // [d]: weight for the target d - 2 pixels to the left / above
   const uint32_t p0 = uint32_t(base / jc.S), p1 = uint32_t((base + n) / jc.S);
-  const uint32_t total = uint32_t(nrows) * jc.W;
-  const float neg_clamp = -0.1f;
-  const uint32_t sub = threadIdx.x & uint32_t(G - 1);
-  const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~uint32_t(G - 1)));
-  const uint32_t groups = (gridDim.x * blockDim.x) / G;
-  // Every lane of a group has the same T, so a group runs its loop together.
-  for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G; t < total; t += groups) {
-    const int tx = int(t % jc.W), ty = ty0 + int(t / jc.W);
-    // The target pixel on the film; the samples of the pattern pixels within
-    // the filter's reach add to it.
-    const int fx = jc.OX + tx, fy = jc.OY + ty;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float wacc = 0.f;
-    for (int dy = -2; dy <= 2; dy++) {
-      const int row = fy + dy - jc.PY;
-      if (row < 0 || row >= int(jc.PH)) continue;
-      for (int dx = -2; dx <= 2; dx++) {
-        const int col = fx + dx - jc.PX;
-        if (col < 0 || col >= int(jc.PW)) continue;
-        const uint32_t pidx = uint32_t(row) * jc.PW + uint32_t(col);
-        if (pidx < p0 || pidx >= p1) continue;
-        const uint32_t pbase = (pidx - p0) * jc.S;
-        for (uint32_t k = sub; k < jc.S; k += G) {
-          float2 j = jit[pbase + k];
-          float sx = float(fx + dx) + j.x, sy = float(fy + dy) + j.y;
-          float w = mitchell1(sx - (float(fx) + 0.5f)) * mitchell1(sy - (float(fy) + 0.5f));
-          if (w == 0.f) continue;
-          float4 r = rad[pbase + k];
-          // Tint (radiance, alpha) stores alpha-scaled colour (color/tint.h:45-49)
-          float cr = r.x * r.w * w, cg = r.y * r.w * w, cb = r.z * r.w * w, ca = r.w * w;
-          if (w < 0.f) {
-            float mc = fminf(cr, fminf(cg, cb));
-            if (mc < neg_clamp) {
-              float sc = neg_clamp / mc;
-              w *= sc;
-              cr *= sc; cg *= sc; cb *= sc; ca *= sc;
-            }
-          }
-          acc.x += cr; acc.y += cg; acc.z += cb; acc.w += ca;
-          wacc += w;
-        }
+  const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
+  const int x0 = int(blockIdx.y) * kSplatW, y0 = ty0 + int(blockIdx.z) * kSplatH;
+  float4 acc[kSplatRows];
+  float wacc[kSplatRows];
+#pragma unroll
+  for (int r = 0; r < kSplatRows; r++) {
+    acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    wacc[r] = 0.f;
+  }
+  // This thread's pattern pixels around the tile, from the wave's first on.
+  constexpr int kRounds = (kHalo + 32 * kSplatWarps - 1) / (32 * kSplatWarps);
+  uint32_t pix[kRounds];
+#pragma unroll
+  for (int q = 0; q < kRounds; q++) {
+    const int i = int(threadIdx.x) + q * 32 * kSplatWarps;
+    const int pc = jc.OX + x0 - 2 + i % kHaloW - jc.PX, pr = jc.OY + y0 - 2 + i / kHaloW - jc.PY;
+    const uint32_t pidx = uint32_t(pr) * jc.PW + uint32_t(pc);
+    const bool in = i < kHalo && pc >= 0 && pc < int(jc.PW) && pr >= 0 && pr < int(jc.PH) && pidx >= p0 && pidx < p1;
+    pix[q] = in ? pidx - p0 : ~0u;
+  }
+  for (uint32_t k = blockIdx.x; k < jc.S; k += gridDim.x) {
+    // All loads of the slice first: their latency is paid once.
+    bool wild = false;   // a colour that is not finite
+    float2 jq[kRounds];
+    float4 rq[kRounds];
+#pragma unroll
+    for (int q = 0; q < kRounds; q++) {
+      jq[q] = make_float2(0.f, 0.f);
+      rq[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (pix[q] != ~0u) {
+        const size_t at = size_t(pix[q]) * jc.S + k;
+        jq[q] = jit[at];
+        rq[q] = rad[at];
       }
     }
 #pragma unroll
-    for (int off = G / 2; off > 0; off >>= 1) {
-      acc.x += __shfl_xor_sync(gmask, acc.x, off);
-      acc.y += __shfl_xor_sync(gmask, acc.y, off);
-      acc.z += __shfl_xor_sync(gmask, acc.z, off);
-      acc.w += __shfl_xor_sync(gmask, acc.w, off);
-      wacc += __shfl_xor_sync(gmask, wacc, off);
+    for (int q = 0; q < kRounds; q++) {
+      const int i = int(threadIdx.x) + q * 32 * kSplatWarps;
+      if (i >= kHalo) break;
+      const float4 r = rq[q];
+      // Tint (radiance, alpha) stores alpha-scaled colour (color/tint.h:45-49)
+      const float4 c = make_float4(r.x * r.w, r.y * r.w, r.z * r.w, r.w);
+      col[i] = c;
+      wlo[i] = -0.1f / fmaxf(fmaxf(c.x, fmaxf(c.y, c.z)), 0.f);   // (-inf where nothing is positive)
+      wild |= !(fabsf(c.x) < INFINITY && fabsf(c.y) < INFINITY && fabsf(c.z) < INFINITY && fabsf(c.w) < INFINITY);
+      const int px = jc.OX + x0 - 2 + i % kHaloW, py = jc.OY + y0 - 2 + i / kHaloW;
+      const float sx = float(px) + jq[q].x, sy = float(py) + jq[q].y;
+#pragma unroll
+      for (int d = 0; d < 5; d++) {
+        wx[d][i] = pix[q] != ~0u ? mitchell1(sx - (float(px - (d - 2)) + 0.5f)) : 0.f;
+        wy[d][i] = mitchell1(sy - (float(py - (d - 2)) + 0.5f));
+      }
     }
-    if (sub == 0) {
-      const size_t o = size_t(ty) * jc.W + size_t(tx);
-      float4 a = accum[o];
-      accum[o] = make_float4(a.x + acc.x, a.y + acc.y, a.z + acc.z, a.w + acc.w);
-      wsum[o] += wacc;
+    // A zero weight is skipped where an infinite colour could meet it.
+    auto add = [&](auto guard) {
+#pragma unroll 1
+      for (int dx = 0; dx < 5; dx++) {
+#pragma unroll
+        for (int h = 0; h < kSplatRows + 4; h++) {
+          const int i = (group * kSplatRows + h) * kHaloW + lane + dx;
+          const float4 c = col[i];
+          const float ux = wx[dx][i], lo = wlo[i];
+#pragma unroll
+          for (int r = 0; r < kSplatRows; r++) {
+            if (h < r || h > r + 4) continue;
+            const float w = fmaxf(ux * wy[h - r][i], lo);
+            if (guard() && w == 0.f) continue;
+            acc[r].x = fmaf(c.x, w, acc[r].x);
+            acc[r].y = fmaf(c.y, w, acc[r].y);
+            acc[r].z = fmaf(c.z, w, acc[r].z);
+            acc[r].w = fmaf(c.w, w, acc[r].w);
+            wacc[r] += w;
+          }
+        }
+      }
+    };
+    if (__syncthreads_or(wild)) add(std::true_type{});
+    else add(std::false_type{});
+    __syncthreads();
+  }
+  const int tx = x0 + lane;
+  if (tx >= int(jc.W)) return;
+#pragma unroll
+  for (int r = 0; r < kSplatRows; r++) {
+    const int ty = y0 + group * kSplatRows + r;
+    if (ty >= ty0 + nrows) break;
+    const size_t o = size_t(ty) * jc.W + size_t(tx);
+    if (ATOMIC) {
+      float *a = reinterpret_cast<float *>(accum + o);
+      atomicAdd(a, acc[r].x);
+      atomicAdd(a + 1, acc[r].y);
+      atomicAdd(a + 2, acc[r].z);
+      atomicAdd(a + 3, acc[r].w);
+      atomicAdd(wsum + o, wacc[r]);
+    } else {
+      const float4 a = accum[o];
+      accum[o] = make_float4(a.x + acc[r].x, a.y + acc[r].y, a.z + acc[r].z, a.w + acc[r].w);
+      wsum[o] += wacc[r];
     }
   }
 }
 
-// The splat with the lane group that fits S samples per pixel.
+// The splat of NROWS target rows from TY0 on.
 void launch_splat(const JobConsts &jc, uint64_t base, uint32_t n, const float4 *rad, const float2 *jit,
-                  float4 *accum, float *wsum, int ty0, int nrows, uint32_t grid256, cudaStream_t st) {
-  if (jc.S >= 32) k_splat<32><<<grid256, 256, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
-  else if (jc.S > 8) k_splat<16><<<grid256, 256, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
-  else if (jc.S > 4) k_splat<8><<<grid256, 256, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
-  else if (jc.S > 2) k_splat<4><<<grid256, 256, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
-  else if (jc.S > 1) k_splat<2><<<grid256, 256, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
-  else k_splat<1><<<grid256, 256, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
+                  float4 *accum, float *wsum, int ty0, int nrows, cudaStream_t st) {
+  const uint32_t tx = (jc.W + kSplatW - 1) / kSplatW, ty = (uint32_t(nrows) + kSplatH - 1) / kSplatH;
+  // Five blocks fit an SM: split the samples until the blocks fill the device
+  // three times over, which leaves a small last round (853x479 at 9 samples:
+  // 164 us filled once, 145 us three times, 157 us twelve times).
+  const uint64_t tiles = uint64_t(tx) * ty, want = uint64_t(num_sms()) * 5 * 3;
+  uint32_t split = tiles >= want ? 1u : uint32_t(want / tiles);
+  split = split < jc.S ? split : jc.S;
+  const auto kernel = split > 1u ? k_splat<true> : k_splat<false>;
+  kernel<<<dim3(split, tx, ty), 32 * kSplatWarps, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
 }
 
 // ImageSampledOutput::set_raw_min_y row flush (image/image-sampled-output.cc:79-123).
@@ -789,7 +856,7 @@ cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, 
     const int ty0 = a0 < 0 ? 0 : a0, ty1 = a1 > int(jc.H) - 1 ? int(jc.H) - 1 : a1;
     if (ty1 >= ty0) {
       if (prof) prof->begin(st, RenderProfile::OTHER);
-      launch_splat(jc, base, n, wb.rad, P.jit, accum, wsum, ty0, ty1 - ty0 + 1, grid256, st);
+      launch_splat(jc, base, n, wb.rad, P.jit, accum, wsum, ty0, ty1 - ty0 + 1, st);
       if (prof) prof->end(st);
       nl++;
     }
@@ -814,7 +881,7 @@ cudaError_t splat_job(const JobConsts &jc, const float4 *rad, const float2 *jit,
   if (e == cudaSuccess) e = cudaMemsetAsync(wsum, 0, npix * sizeof(float), st);
   if (e != cudaSuccess) return e;
   const uint32_t grid256 = uint32_t(num_sms()) * 8;
-  launch_splat(jc, 0, uint32_t(total), rad, jit, accum, wsum, 0, int(jc.H), grid256, st);
+  launch_splat(jc, 0, uint32_t(total), rad, jit, accum, wsum, 0, int(jc.H), st);
   k_resolve<<<grid256, 256, 0, st>>>(uint32_t(npix), accum, wsum, out_rgb);
   return cudaGetLastError();
 }
