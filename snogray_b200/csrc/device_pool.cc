@@ -1,0 +1,123 @@
+// device_pool.cc -- the kept device blocks behind device_pool.h.
+
+#include "device_pool.h"
+
+#include <cuda_runtime.h>
+
+#include <map>
+#include <mutex>
+#include <utility>
+
+#include "scene.h"
+
+namespace snog {
+
+namespace {
+
+struct Block {
+  int device;
+  size_t size;
+};
+
+struct Pool {
+  std::mutex mu;
+  std::map<void *, Block> blocks;                           // every block of the pool
+  std::multimap<std::pair<int, size_t>, void *> kept;       // those not in use, by device and size
+  size_t kept_bytes = 0;
+};
+
+// Never destroyed: blocks may be given back while the process ends.
+Pool &pool() {
+  static Pool *p = new Pool;
+  return *p;
+}
+
+// N rounded up to an eighth of its power of two, at least 4096.
+size_t size_class(size_t n) {
+  if (n <= 4096) return 4096;
+  size_t p = 1;
+  while (p <= n / 2) p <<= 1;
+  const size_t step = p / 8;
+  return (n + step - 1) / step * step;
+}
+
+void trim_locked(Pool &P) {
+  for (auto &k : P.kept) {
+    cudaFree(k.second);
+    P.blocks.erase(k.second);
+  }
+  P.kept.clear();
+  P.kept_bytes = 0;
+}
+
+}  // namespace
+
+void *pool_get(size_t n) {
+  Pool &P = pool();
+  int dev = 0;
+  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  const size_t want = size_class(n);
+  std::lock_guard<std::mutex> lk(P.mu);
+  auto it = P.kept.lower_bound({dev, want});
+  if (it != P.kept.end() && it->first.first == dev && it->first.second <= want + want / 4) {
+    void *p = it->second;
+    P.kept_bytes -= it->first.second;
+    P.kept.erase(it);
+    return p;
+  }
+  void *p = nullptr;
+  cudaError_t e = cudaMalloc(&p, want);
+  if (e == cudaErrorMemoryAllocation && P.kept_bytes) {
+    cudaGetLastError();
+    trim_locked(P);
+    e = cudaMalloc(&p, want);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    throw Error{e == cudaErrorMemoryAllocation ? SNOG_ENOMEM : SNOG_ECUDA,
+                std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+  }
+  try {
+    P.blocks[p] = Block{dev, want};
+  } catch (...) {
+    cudaFree(p);
+    throw;
+  }
+  return p;
+}
+
+void pool_put(void *p) {
+  if (!p) return;
+  Pool &P = pool();
+  std::lock_guard<std::mutex> lk(P.mu);
+  auto it = P.blocks.find(p);
+  if (it == P.blocks.end()) return;
+  const Block b = it->second;
+  if (P.kept_bytes + b.size <= kPoolKeep) {
+    try {
+      P.kept.insert({{b.device, b.size}, p});
+      P.kept_bytes += b.size;
+      return;
+    } catch (...) {   // no room to remember it: free it
+    }
+  }
+  cudaFree(p);
+  P.blocks.erase(it);
+}
+
+void pool_trim() {
+  Pool &P = pool();
+  std::lock_guard<std::mutex> lk(P.mu);
+  trim_locked(P);
+}
+
+bool device_idle(int device) {
+  int cur = 0;
+  if (cudaGetDevice(&cur) != cudaSuccess) return false;
+  if (cur != device && cudaSetDevice(device) != cudaSuccess) return false;
+  const bool ok = cudaDeviceSynchronize() == cudaSuccess;
+  if (cur != device) cudaSetDevice(cur);
+  return ok;
+}
+
+}  // namespace snog

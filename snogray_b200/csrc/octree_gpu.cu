@@ -320,18 +320,32 @@ __global__ void k_scatter_inverse(const uint32_t *perm, uint32_t n, uint32_t *in
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) inv[perm[i]] = i;
 }
 
-// Temporary device memory of one build, freed on every exit path.
+// Temporary device memory of one build, given back on every exit path: cut
+// from a few blocks, each twice the one before, of sizes that any build asks
+// the pool for.
 struct Scratch {
   std::vector<void *> p;
+  char *at = nullptr;
+  size_t left = 0, next = size_t(16) << 20;
   template <class T>
   T *get(size_t n) {
-    void *q = nullptr;
-    check_cuda(cudaMalloc(&q, n ? n * sizeof(T) : 16), "octree build scratch");
-    p.push_back(q);
-    return static_cast<T *>(q);
+    const size_t need = ((n ? n * sizeof(T) : 16) + 255) & ~size_t(255);
+    if (need > left) {
+      while (next < need) next *= 2;
+      p.reserve(p.size() + 1);
+      at = static_cast<char *>(pool_get(next));
+      p.push_back(at);
+      left = next;
+      next *= 2;
+    }
+    char *q = at;
+    at += need;
+    left -= need;
+    return reinterpret_cast<T *>(q);
   }
   ~Scratch() {
-    for (void *q : p) cudaFree(q);
+    cudaStreamSynchronize(nullptr);   // the build's stream; a failed build may still be running
+    for (void *q : p) pool_put(q);
   }
 };
 

@@ -31,14 +31,9 @@ void check_render_flags(uint32_t flags) {
 }
 
 void *DeviceArena::alloc(size_t n) {
-  void *p = nullptr;
-  size_t sz = n ? (n + 255) & ~size_t(255) : 256;
-  cudaError_t e = cudaMalloc(&p, sz);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    throw Error{e == cudaErrorMemoryAllocation ? SNOG_ENOMEM : SNOG_ECUDA,
-                std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-  }
+  const size_t sz = n ? (n + 255) & ~size_t(255) : 256;
+  blocks.reserve(blocks.size() + 1);
+  void *p = pool_get(sz);
   blocks.push_back(p);
   bytes += sz;
   return p;
@@ -51,7 +46,7 @@ void *DeviceArena::upload(const void *src, size_t n) {
 }
 
 void DeviceArena::release() {
-  for (void *p : blocks) cudaFree(p);
+  for (void *p : blocks) pool_put(p);
   blocks.clear();
   bytes = 0;
 }
@@ -519,6 +514,7 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
     D.env_row_cdf = dev_upload(A, row_cdf);
     D.env_col_cdf = dev_upload(A, col_cdf);
   } catch (...) {
+    device_idle(S.device);
     A.release();
     throw;
   }

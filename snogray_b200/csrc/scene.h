@@ -4,11 +4,13 @@
 #define SNOG_SCENE_H
 
 #include <cstdint>
+#include <exception>
 #include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/snogray_b200.h"
+#include "device_pool.h"
 #include "octree_build.h"
 #include "snog_common.h"
 #include "wavefront.h"
@@ -30,9 +32,9 @@ struct RenderCache {
 struct DeviceArena {
   std::vector<void *> blocks;
   uint64_t bytes = 0;
-  void *alloc(size_t n);           // throws CudaError on failure
+  void *alloc(size_t n);           // throws Error on failure
   void *upload(const void *src, size_t n);
-  void release();
+  void release();                  // to the pool: the device must be idle
 };
 
 struct SceneImpl {
@@ -90,19 +92,17 @@ struct Error {
 void check_cuda(int err, const char *what);   // throws Error{SNOG_ECUDA}
 
 // RAII device buffer for per-call temporaries (at least 16 bytes, so a
-// zero-length request still yields a valid pointer).
+// zero-length request still yields a valid pointer), from the pool.  The call
+// waits for its work before it returns; one that ends by an exception may not
+// have, and waits here.
 struct DevBuf {
   void *p = nullptr;
-  explicit DevBuf(size_t n) {
-    if (n == 0) n = 16;
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      throw Error{e == cudaErrorMemoryAllocation ? SNOG_ENOMEM : SNOG_ECUDA,
-                  std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-    }
+  int device = 0;
+  explicit DevBuf(size_t n) : p(pool_get(n ? n : 16)) { cudaGetDevice(&device); }
+  ~DevBuf() {
+    if (std::uncaught_exceptions()) device_idle(device);
+    pool_put(p);
   }
-  ~DevBuf() { cudaFree(p); }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
   template <class T>

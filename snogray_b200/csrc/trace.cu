@@ -143,9 +143,9 @@ uint32_t probe_pair_lists(const DevScene &s) {
     rays[5 * size_t(n) + i] = z;
     rays[6 * size_t(n) + i] = INFINITY;
   }
-  char *block = nullptr;
   const size_t rb = rays.size() * 4, pb = size_t(n) * 4;
-  check_cuda(cudaMalloc(&block, rb + pb + 64), "probe buffers");
+  const DevBuf buf(rb + pb + 64);
+  char *block = buf.as<char>();
   unsigned long long cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   cudaError_t e = cudaMemcpy(block, rays.data(), rb, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(block + rb + pb, 0, 64);
@@ -156,7 +156,6 @@ uint32_t probe_pair_lists(const DevScene &s) {
                            nullptr, nullptr);
   }
   if (e == cudaSuccess) e = cudaMemcpy(cnt, block + rb + pb, 64, cudaMemcpyDeviceToHost);
-  cudaFree(block);
   check_cuda(e, "list probe");
   // cnt[0]: node visits, cnt[1]: primitive tests of the closest-hit queries
   return cnt[1] > 5 * cnt[0] / 2 ? 1u : 0u;
