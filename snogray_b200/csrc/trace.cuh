@@ -407,10 +407,11 @@ struct Traversal {
     const bool slow = octant & kSlowSlab;
     bool open = true;
     const bool any_query = ANY == kAnyOnly || (ANY == kMixed && (octant & kAnyHit));
-    if ((octant & kGateFlag) && any_query) {
+    if (ANY == kAnyOnly || ((octant & kGateFlag) && any_query)) {
       // An any-hit query's extent never changes, so an entry with a parent
       // gate passed the very gate and cull it would be given now when it
       // was pushed (or entered): the call happens and the node is open.
+      // (The root of an any-hit kernel's rays passed its cull at the start.)
       if (COUNT) cnt.nodes++;
     } else {
       // The cull decides alone where bounds are finite: it closes whatever the
@@ -524,7 +525,8 @@ struct Traversal {
       sp--;
     }
     node = first + __popc(bits & ((1u << (cb ^ (octant & 7u))) - 1u));
-    octant = (octant & (kGateFlag - 1u)) | kGateFlag | (cb << kGateShift);
+    if (COUNT || slow) octant = (octant & (kGateFlag - 1u)) | kGateFlag | (cb << kGateShift);
+    else if (ANY == kMixed) octant |= kGateFlag;
     // The far half starts at mid; either half ends half an extent after it starts.
     if (cb & 4) lo.x = __fadd_rn(lo.x, half.x);
     if (cb & 2) lo.y = __fadd_rn(lo.y, half.y);
@@ -575,8 +577,11 @@ __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool any, Trace
   uint32_t incl = np;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const uint32_t v = __shfl_up_sync(kFull, incl, off);
-    if (lane >= uint32_t(off)) incl += v;
+    // incl += its value OFF lanes below, where there is such a lane (the shuffle's own predicate says).
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .u32 v;\n shfl.sync.up.b32 v|p, %0, %1, 0, 0xffffffff;\n @p add.u32 %0, %0, v;\n}"
+        : "+r"(incl)
+        : "r"(off));
   }
   const uint32_t excl = incl - np;
   const uint32_t total = __shfl_sync(kFull, incl, 31);
@@ -760,7 +765,10 @@ struct RayDispenser {
 // a third 16-byte part per stack record and a vote on every refill, with
 // the ring of 4 records that the smaller ones make room for: terrain frame
 // 201.9 -> 190.9 ms, 16M rays in 1M triangles 17.6 -> 16.4 ms, 200k-triangle
-// soup 19.8 -> 17.7 ms.
+// soup 19.8 -> 17.7 ms.  One reduction for pending entries and waiting lanes,
+// the refill threshold in a register, the scan's additions under the shuffle's
+// own predicate, no gate word and no entry test where a kernel does not
+// need them: terrain frame 170.0 -> 167.0 ms.
 template <int STACK, int ANY, int PER, bool COUNT, class Start, class Done>
 __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, TraceCounters &cnt, Start start,
                                            Done done) {
@@ -775,18 +783,28 @@ __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, Trac
   // Idle lanes take new rays only once refill_min of those that may are idle:
   // a ray start (queue loads, root slab set-up, ray slot) then runs on several
   // lanes at once instead of on one or two every iteration.
+  // (The ray-batch kernel has no register for the threshold: 16M rays 15.7 ms
+  // without, 16.4 with.)
+  uint32_t refill_at = 32u - disp.limit + (refill_min(ANY) < disp.limit ? refill_min(ANY) : disp.limit);
   for (;;) {
     const uint32_t idle = __ballot_sync(0xffffffffu, ray == RayDispenser::kIdle);
-    if (disp.limit == 0u) {
-      if (idle == 0xffffffffu) break;
-    } else if (__popc(idle) + disp.limit >= 32u + (refill_min(ANY) < disp.limit ? refill_min(ANY) : disp.limit)) {
+    if (ANY == kMixed)
+      refill_at = disp.limit ? 32u - disp.limit + (refill_min(ANY) < disp.limit ? refill_min(ANY) : disp.limit) : 33u;
+    if (uint32_t(__popc(idle)) >= refill_at) {
       const uint32_t got =
           disp.fetch(dispenser, n, ray == RayDispenser::kIdle && (threadIdx.x & 31u) < disp.limit);
+      if (disp.limit == 0u) refill_at = 33u;   // never again
       if (got != RayDispenser::kIdle) {
         ray = got;
         start(ray, tr, any);
         if (any) tr.octant |= kAnyHit;
+        if (ANY == kAnyOnly && tr.have && !slab_open(tr.t0, tr.t1, tr.lo, tr.hi)) {
+          if (COUNT) cnt.nodes++;
+          tr.have = false;
+        }
       }
+    } else if (idle == 0xffffffffu) {
+      break;
     }
     // Visit nodes only while the warp's pending list entries would not fill
     // a round: list rounds run full, node steps run with more lanes at once.
@@ -800,8 +818,10 @@ __device__ __forceinline__ void trace_loop(uint32_t *dispenser, uint32_t n, Trac
     bool round = true;
     if (ANY == kClosestOnly) {
       const uint32_t pend2 = tr.lend - tr.lp;
-      const uint32_t pending2 = __reduce_add_sync(0xffffffffu, pend2 < 32u ? pend2 : 32u);
-      round = pending2 >= kRoundMin || __popc(__ballot_sync(0xffffffffu, tr.have && pend2 == 0u)) <= kFewSteps;
+      // Pending entries (at most 1024) and, above them, lanes that could visit a node.
+      const uint32_t both = __reduce_add_sync(
+          0xffffffffu, pend2 ? (pend2 < 32u ? pend2 : 32u) : tr.have ? 1u << 16 : 0u);
+      round = (both & 0xffffu) >= kRoundMin || both < (kFewSteps + 1u) << 16;
     }
     const bool stop = round && list_round<STACK, ANY, PER>(tr, any, cnt);
     if (ray != RayDispenser::kIdle && (stop || tr.finished())) {
