@@ -177,7 +177,7 @@ static void render_into(SceneImpl &S, const SnogCamera &cam, const SnogRenderPar
   WaveBuffers wave = rc.wb;   // the pool may be larger than this job's wave
   wave.wave_cap = cap;
   cudaError_t e = render_job(S.dev, jc, wave, rc.accum, rc.wsum, d_out ? d_out : rc.out, st, &waves,
-                             &launches, profile ? &prof : nullptr, count);
+                             &launches, profile ? &prof : nullptr, count, &pool.side);
   if (e == cudaSuccess && !d_out)
     e = cudaMemcpyAsync(h_out, rc.out, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaEventRecord(pool.done, st);

@@ -71,10 +71,8 @@ __global__ void k_e_plan(EngineCtl *ctl, const WorkItem *ring, uint32_t R, uint3
   ctl->paths_started += n_new;
   ctl->qcount[cur] = n_cur + take + uint32_t(n_new);
   ctl->qcount[cur ^ 1u] = 0;
-  ctl->scount = 0;
   ctl->dcount = 0;
   ctl->disp_closest = 0;
-  ctl->disp_shadow = 0;
 }
 
 // New camera paths for tickets [regen_start, regen_start + regen_n).
@@ -222,6 +220,10 @@ __global__ void __launch_bounds__(BLOCK, shade_blocks(BLOCK)) k_e_shade(EngineCt
                                                  unsigned long long *job_done, unsigned long long *job_spawned,
                                                  EQ sp, uint32_t sp_cap) {
   const uint32_t n = ctl->qcount[cur];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->scount = 0;        // the last iteration's shadow rays are traced: the
+    ctl->disp_shadow = 0;   // queue starts empty, as does its dispenser
+  }
   uint32_t *count_out = &ctl->qcount[cur ^ 1u];
   const uint32_t lane = threadIdx.x & 31u;
   const ShadeItems<BLOCK> items(n);
@@ -584,7 +586,7 @@ void launch_iteration(cudaStream_t st, EngineCtl *ctl, const WorkItem *ring, uin
                       uint32_t cur, const EngineJobDev *jobs, const DevScene *scenes, EQ qc, EQ qn,
                       uint32_t *hit_ref, float *hit_t, EDL dl, ESQ sq, unsigned long long *job_done,
                       unsigned long long *job_spawned, EQ sp, uint32_t sp_cap, bool direct, bool long_run,
-                      const cudaEvent_t *ev) {
+                      const cudaEvent_t *ev, ShadowStream *side, bool first) {
   const uint32_t sms = uint32_t(num_sms());
   if (ev) cudaEventRecord(ev[0], st);
   k_e_plan<<<1, 1, 0, st>>>(ctl, ring, R, N, cur, sp_cap);
@@ -593,6 +595,8 @@ void launch_iteration(cudaStream_t st, EngineCtl *ctl, const WorkItem *ring, uin
   k_e_closest<STACK, PER><<<resident_grid(k_e_closest<STACK, PER>, kTraceBlock), kTraceBlock, 0, st>>>(
       ctl, cur, jobs, scenes, qc, hit_ref, hit_t);
   if (ev) cudaEventRecord(ev[2], st);
+  // The last iteration's shadow rays add to the radiance that shading reads.
+  if (side && !first) cudaStreamWaitEvent(st, side->done, 0);
   auto shading = [&](auto d, auto block) {
     constexpr int kBlock = block();
     const uint32_t grid = sms * (kBlock == kLongBlock ? 1u : 12u);
@@ -605,7 +609,13 @@ void launch_iteration(cudaStream_t st, EngineCtl *ctl, const WorkItem *ring, uin
   if (direct) long_run ? shading(std::true_type{}, long_block) : shading(std::true_type{}, short_block);
   else long_run ? shading(std::false_type{}, long_block) : shading(std::false_type{}, short_block);
   if (ev) cudaEventRecord(ev[3], st);
-  k_e_shadow<STACK><<<resident_grid(k_e_shadow<STACK>, kTraceBlock), kTraceBlock, 0, st>>>(ctl, scenes, sq);
+  const cudaStream_t on = side ? side->st : st;
+  if (side) {
+    cudaEventRecord(side->lit, st);
+    cudaStreamWaitEvent(on, side->lit, 0);
+  }
+  k_e_shadow<STACK><<<resident_grid(k_e_shadow<STACK>, kTraceBlock), kTraceBlock, 0, on>>>(ctl, scenes, sq);
+  if (side) cudaEventRecord(side->done, on);
   if (ev) cudaEventRecord(ev[4], st);
 }
 
@@ -670,6 +680,7 @@ Engine::Engine(const EngineConfigHost &cfg, cudaStream_t stream) : cfg_(cfg) {
     check_cuda(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "stream");
     own_stream_ = true;
   }
+  check_cuda(shadow_stream_.create(), "shadow stream");
   const size_t N = cfg_.slots, L = cfg_.max_lights ? cfg_.max_lights : 1;
   size_t off = 0;
   auto take = [&](size_t b) {
@@ -743,6 +754,9 @@ Engine::~Engine() {
   cudaFreeHost(done_host_);
   cudaFreeHost(staging_);
   for (cudaEvent_t e : events_) cudaEventDestroy(e);
+  if (shadow_stream_.lit) cudaEventDestroy(shadow_stream_.lit);
+  if (shadow_stream_.done) cudaEventDestroy(shadow_stream_.done);
+  if (shadow_stream_.st) cudaStreamDestroy(shadow_stream_.st);
   if (own_stream_) cudaStreamDestroy(stream_);
 }
 
@@ -798,6 +812,9 @@ void Engine::launch_iterations(bool direct, bool pair, bool long_run) {
   for (int k = 0; k < 2; k++) q[k] = EQ{q_o_[k], q_d_[k], q_thr_[k], q_rad_[k], q_meta_[k]};
   ESQ sq{s_o_, s_d_, s_c_, s_tgt_};
   const uint32_t n_iter = 2 * cfg_.iters_per_launch;
+  // Shadow rays beside the next iteration's closest hits, but for the profile,
+  // whose events bracket launches of one stream.
+  ShadowStream *side = profile_on_ ? nullptr : &shadow_stream_;
   if (profile_on_ && events_.size() < 5 * size_t(n_iter)) {
     while (events_.size() < 5 * size_t(n_iter)) {
       cudaEvent_t e;
@@ -812,7 +829,7 @@ void Engine::launch_iterations(bool direct, bool pair, bool long_run) {
   launch_iteration<S, P>(stream_, ctl_, ring_, cfg_.ring_items, cfg_.slots, cur, jobs_dev_, scenes_dev_, q[cur], \
                          q[cur ^ 1], hit_ref_, hit_t_, EDL{d_idx_, d_tgt_}, sq, job_done_,                      \
                          job_done_ + cfg_.max_jobs, EQ{sp_o_, sp_d_, sp_thr_, sp_rad_, sp_meta_}, sp_cap_,     \
-                         direct, long_run, ev)
+                         direct, long_run, ev, side, it == 0)
     switch (graph_stack_ * 2 + (pair ? 1 : 0)) {
       case 64: SNOG_ITER(32, 1); break;
       case 65: SNOG_ITER(32, 2); break;
@@ -825,6 +842,7 @@ void Engine::launch_iterations(bool direct, bool pair, bool long_run) {
     }
 #undef SNOG_ITER
   }
+  if (side) check_cuda(cudaStreamWaitEvent(stream_, side->done, 0), "shadow join");
 }
 
 void Engine::build_graph(bool direct, bool pair, bool long_run) {

@@ -11,7 +11,9 @@
 //                and roulette; surviving paths go to the other queue,
 //                finished ones write their radiance to their job's result
 //   k_e_shadow   any-hit for the shadow rays; unoccluded ones add their
-//                contribution to the path's next-queue entry or result
+//                contribution to the path's next-queue entry or result; on a
+//                branch of its own, beside the next iteration's plan, regen
+//                and closest, and joined before its shading
 // The host admits jobs (device-memory budget), pushes their items into the
 // ring round-robin across jobs (so jobs that arrive later interleave with
 // running ones), launches the graph, and gathers-and-filters each job's
@@ -221,6 +223,7 @@ class Engine {
   // [with the direct integrator's shading][closest-hit rounds in pairs][shading in long blocks]
   cudaGraphExec_t graph_[2][2][2] = {};
   int graph_stack_ = 0;
+  ShadowStream shadow_stream_;
   // device buffers
   void *block_ = nullptr;
   float4 *q_o_[2], *q_d_[2], *q_thr_[2], *q_rad_[2];

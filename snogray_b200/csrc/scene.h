@@ -60,6 +60,7 @@ struct SceneImpl {
 struct RenderPool {
   std::mutex mu;
   RenderCache rc;
+  ShadowStream side;
   cudaEvent_t done = nullptr;
 };
 RenderPool &render_pool(int device);

@@ -14,7 +14,9 @@
 //     k_direct               direct lighting with MIS of the listed
 //                            vertices (emits shadow rays)
 //     k_trace_shadow         any-hit for the shadow rays; unoccluded ones add
-//                            their contribution to the path's radiance
+//                            their contribution to the path's radiance; on a
+//                            stream of its own, beside the next bounce's
+//                            k_trace_closest, and joined before its k_shade
 //   k_splat                  Mitchell filter gather of the wave's samples
 //                            into the image accumulator
 // and finally k_resolve divides by the filter weight
@@ -116,10 +118,8 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_clo
                                                        unsigned long long *stats) {
   const uint32_t n = counters[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    counters[cur ^ 1u] = 0;   // next queue and shadow queue start empty
-    counters[2] = 0;
-    counters[5] = 0;          // shadow kernel's dispenser
-    counters[6] = 0;          // direct-lighting list
+    counters[cur ^ 1u] = 0;   // the next queue and the direct-lighting list start empty
+    counters[6] = 0;
     stats[0] += n;
   }
   TraceCounters c{0, 0, 0};
@@ -146,7 +146,6 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_sha
   const uint32_t n = counters[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     stats[1] += n;
-    stats[6] += counters[6];   // vertices lit this bounce (DirectIllum::sample_all_lights calls)
   }
   TraceCounters c{0, 0, 0};
   trace_loop<STACK, kAnyOnly, 1, COUNT>(
@@ -174,7 +173,11 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene s, JobConsts jc, uint
                                                const uint32_t *hit_ref, const float *hit_t, PathPtrs P,
                                                RayQ qout, DirectL dl) {
   const uint32_t n = counters[cur];
-  if (blockIdx.x == 0 && threadIdx.x == 0) counters[4] = 0;   // next bounce's dispenser
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    counters[4] = 0;   // next bounce's dispenser
+    counters[2] = 0;   // the last bounce's shadow rays are traced: the queue
+    counters[5] = 0;   // starts empty, as does its dispenser
+  }
   uint32_t *count_out = counters + (cur ^ 1u);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -308,8 +311,10 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene s, JobConsts jc, uint
 // over a compacted list so escaped and absorbed paths leave no idle lanes.
 __global__ void __launch_bounds__(128, 6) k_direct(DevScene s, JobConsts jc, uint64_t base, uint32_t bounce,
                                                 RayQ qin, uint32_t *counters, const uint32_t *hit_ref,
-                                                const float *hit_t, DirectL dl, ShadowQ sq) {
+                                                const float *hit_t, DirectL dl, ShadowQ sq,
+                                                unsigned long long *stats) {
   const uint32_t n = counters[6];
+  if (blockIdx.x == 0 && threadIdx.x == 0) stats[6] += n;   // DirectIllum::sample_all_lights calls
   uint32_t *count_sq = counters + 2;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -620,7 +625,7 @@ __global__ void __launch_bounds__(256) k_resolve(uint32_t npix, const float4 *ac
 
 template <int STACK, bool COUNT>
 void launch_bounce(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, uint64_t base, uint32_t b,
-                   uint32_t cur, uint32_t grid128, cudaStream_t st, RenderProfile *prof) {
+                   uint32_t cur, uint32_t grid128, cudaStream_t st, RenderProfile *prof, ShadowStream *side) {
   RayQ qin{wb.q_o[cur], wb.q_d[cur], wb.q_path[cur]};
   RayQ qout{wb.q_o[cur ^ 1], wb.q_d[cur ^ 1], wb.q_path[cur ^ 1]};
   ShadowQ sq{wb.s_o, wb.s_d, wb.s_c};
@@ -632,10 +637,19 @@ void launch_bounce(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, uint
   closest<<<resident_grid(closest, kTraceBlock), kTraceBlock, 0, st>>>(s, qin, wb.counters, cur, wb.hit_ref,
                                                                        wb.hit_t, wb.stats);
   if (prof) prof->end(st), prof->begin(st, RenderProfile::SHADE);
+  // The last bounce's shadow rays add to the radiance that shading reads.
+  if (side && b) cudaStreamWaitEvent(st, side->done, 0);
   k_shade<<<grid128, 128, 0, st>>>(s, jc, base, b, qin, wb.counters, cur, wb.hit_ref, wb.hit_t, P, qout, dl);
-  k_direct<<<grid128, 128, 0, st>>>(s, jc, base, b, qin, wb.counters, wb.hit_ref, wb.hit_t, dl, sq);
+  k_direct<<<grid128, 128, 0, st>>>(s, jc, base, b, qin, wb.counters, wb.hit_ref, wb.hit_t, dl, sq,
+                                     wb.stats);
   if (prof) prof->end(st), prof->begin(st, RenderProfile::SHADOW);
-  shadow<<<resident_grid(shadow, kTraceBlock), kTraceBlock, 0, st>>>(s, sq, wb.counters, wb.rad, wb.stats);
+  const cudaStream_t on = side ? side->st : st;
+  if (side) {
+    cudaEventRecord(side->lit, st);
+    cudaStreamWaitEvent(on, side->lit, 0);
+  }
+  shadow<<<resident_grid(shadow, kTraceBlock), kTraceBlock, 0, on>>>(s, sq, wb.counters, wb.rad, wb.stats);
+  if (side) cudaEventRecord(side->done, on);
   if (prof) prof->end(st);
 }
 
@@ -814,14 +828,24 @@ JobConsts make_job(const DevScene &s, const SnogCamera &cam, const SnogRenderPar
   return jc;
 }
 
+cudaError_t ShadowStream::create() {
+  cudaError_t e = cudaSuccess;
+  if (!lit) e = cudaEventCreateWithFlags(&lit, cudaEventDisableTiming);
+  if (e == cudaSuccess && !done) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+  if (e == cudaSuccess && !st) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  return e;
+}
+
 cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, float4 *accum, float *wsum,
                        float *out_rgb, cudaStream_t st, uint32_t *waves, uint32_t *launches,
-                       RenderProfile *prof, bool count) {
+                       RenderProfile *prof, bool count, ShadowStream *side) {
+  if (prof) side = nullptr;   // the profile's events bracket launches of one stream
   const uint64_t npix = uint64_t(jc.W) * jc.H;
   cudaError_t e = cudaMemsetAsync(accum, 0, npix * sizeof(float4), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(wsum, 0, npix * sizeof(float), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(wb.stats, 0, 64, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(wb.counters, 0, 64, st);
+  if (e == cudaSuccess && side) e = side->create();
   if (e != cudaSuccess) return e;
   const int sms = num_sms();
   const uint32_t grid128 = uint32_t(sms) * 12, grid256 = uint32_t(sms) * 8;
@@ -841,8 +865,8 @@ cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, 
     for (uint32_t b = 0; b <= jc.max_len; b++) {
       const uint32_t cur = b & 1u;
       auto bounce = [&](auto stack) {
-        if (prof || count) launch_bounce<stack(), true>(s, jc, wb, base, b, cur, grid128, st, prof);
-        else launch_bounce<stack(), false>(s, jc, wb, base, b, cur, grid128, st, prof);
+        if (prof || count) launch_bounce<stack(), true>(s, jc, wb, base, b, cur, grid128, st, prof, side);
+        else launch_bounce<stack(), false>(s, jc, wb, base, b, cur, grid128, st, prof, side);
       };
       switch (sc) {
         case 32: bounce(std::integral_constant<int, 32>{}); break;
@@ -853,6 +877,7 @@ cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, 
       }
       nl += 4;
     }
+    if (side && (e = cudaStreamWaitEvent(st, side->done, 0)) != cudaSuccess) return e;
     // Output rows reached by this wave's pattern rows (a sample reaches
     // the film rows within 2 of its own).
     const uint32_t p0 = uint32_t(base / jc.S), p1 = uint32_t((base + n) / jc.S);

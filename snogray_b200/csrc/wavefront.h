@@ -29,6 +29,20 @@ struct JobConsts {
   uint32_t integ;           // SNOG_INTEG_PATH or SNOG_INTEG_DIRECT
 };
 
+// The stream on which a bounce's shadow rays are traced beside the next bounce's
+// closest hits, and the events that order the two (created on first use).
+// Each trace launch ends with the few warps that hold its longest rays; side by
+// side the two launches of a bounce end once (853x479 terrain on the wave
+// renderer 8.75 -> 7.43 ms, 256x256x16 terrain on the engine 4.74 -> 4.09, 64x48
+// Cornell 545 -> 456 us; the terrain frame, whose launches are long, 167.0 ->
+// 164.9 ms).  Cutting a wave into two pieces on two streams instead measured
+// 2-6 % on small renders and a loss on large ones.
+struct ShadowStream {
+  cudaStream_t st = nullptr;
+  cudaEvent_t lit = nullptr, done = nullptr;
+  cudaError_t create();
+};
+
 // Device buffers for one wave of paths (sized for wave_cap paths).
 struct WaveBuffers {
   uint64_t wave_cap = 0;
@@ -86,7 +100,8 @@ struct RenderProfile {
 // weight, W*H each; zeroed here) and resolve it to out_rgb (W*H*3 floats,
 // device).  Paths are processed in waves of at most wb.wave_cap.  With PROF,
 // every launch is bracketed by events; with COUNT (or PROF) the traversal
-// counts its node visits and primitive tests into wb.stats[2..5].
+// counts its node visits and primitive tests into wb.stats[2..5].  With SIDE
+// (and no PROF) shadow rays run beside the next bounce's closest hits.
 // Mitchell-filter all TOTAL samples of a finished job (radiance + alpha and
 // camera jitter per path, pattern-pixel-major) into its image: clears
 // accum/wsum, gathers, resolves into out_rgb.
@@ -95,7 +110,7 @@ cudaError_t splat_job(const JobConsts &jc, const float4 *rad, const float2 *jit,
 
 cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, float4 *accum,
                        float *wsum, float *out_rgb, cudaStream_t st, uint32_t *waves, uint32_t *launches,
-                       RenderProfile *prof = nullptr, bool count = false);
+                       RenderProfile *prof = nullptr, bool count = false, ShadowStream *side = nullptr);
 
 }  // namespace snog
 
