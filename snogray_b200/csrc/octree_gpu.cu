@@ -11,12 +11,14 @@
 // node is an ancestor of a list entry; lists are last-in first-out, i.e. in
 // decreasing insertion order; and the final numbering is breadth first with
 // children in octant order.  The only sequential part is the root's growth,
-// which the host replays on the bounding boxes alone (root_start / root_fits
-// / root_grow, shared with the host builder): each run of surfaces inserted
-// under one root (an "epoch") descends from that root, which sits in the
-// final tree below the octants later growths gave it.
+// which the host replays (root_start / root_grow, shared with the host builder)
+// on the boxes that make it grow, each found by a search on the device: each
+// run of surfaces inserted under one root (an "epoch") descends from that
+// root, which sits in the final tree below the octants later growths gave it.
 //
 // Steps (one thread per surface, then per placement, then per node):
+//   0. the triangles' primitive records and bounding boxes from the mesh, in
+//      order, without the degenerate ones; then the root's growth;
 //   1. count, then emit, one record per placement: the node's path as base-8
 //      digits left-aligned in a 128-bit key with the depth in the low byte
 //      (so keys sort in depth-first pre-order, a node before its subtree),
@@ -163,6 +165,70 @@ __device__ __forceinline__ uint32_t epoch_of(const Epoch *ep, uint32_t n_ep, uin
     else hi = mid;
   }
   return lo;
+}
+
+// Triangle i of the mesh: its record (snog_common.h; edges as the reference
+// subtracts them per test, surface/mesh.cc:730-760), its box (BBox += Pos with
+// snogray::min/max, geometry/bbox.h:58-63) and whether the space holds it
+// (degenerate triangles are left out, surface/mesh.cc:833-846), in the host
+// code's single precision steps.
+__global__ void k_oct_triangles(const float *__restrict__ vertices, const uint32_t *__restrict__ triangles, uint32_t n,
+                                float4 *__restrict__ prims, Box3 *__restrict__ boxes, uint32_t *__restrict__ keep) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float p[3][3], e1[3], e2[3];
+    Box3 b;
+    for (int c = 0; c < 3; c++) {
+      const float *v = vertices + 3 * size_t(triangles[3 * size_t(i) + c]);
+      for (int k = 0; k < 3; k++) p[c][k] = v[k];
+    }
+    for (int k = 0; k < 3; k++) {
+      e1[k] = __fsub_rn(p[1][k], p[0][k]);
+      e2[k] = __fsub_rn(p[2][k], p[0][k]);
+      float lo = p[0][k], hi = p[0][k];
+      for (int c = 0; c < 3; c++) {
+        lo = lo < p[c][k] ? lo : p[c][k];
+        hi = hi > p[c][k] ? hi : p[c][k];
+      }
+      b.lo[k] = lo;
+      b.hi[k] = hi;
+    }
+    prims[3 * size_t(i)] = make_float4(p[0][0], p[0][1], p[0][2], float(PRIM_TRI));
+    prims[3 * size_t(i) + 1] = make_float4(e1[0], e1[1], e1[2], 0.f);
+    prims[3 * size_t(i) + 2] = make_float4(e2[0], e2[1], e2[2], 0.f);
+    // e2 x e1 of a left-handed mesh (surface/mesh.h:55), and its squared length.
+    const float cx = __fsub_rn(__fmul_rn(e2[1], e1[2]), __fmul_rn(e2[2], e1[1]));
+    const float cy = __fsub_rn(__fmul_rn(e2[2], e1[0]), __fmul_rn(e2[0], e1[2]));
+    const float cz = __fsub_rn(__fmul_rn(e2[0], e1[1]), __fmul_rn(e2[1], e1[0]));
+    boxes[i] = b;
+    keep[i] =
+        __fadd_rn(__fadd_rn(__fmul_rn(cx, cx), __fmul_rn(cy, cy)), __fmul_rn(cz, cz)) > 0.f ? 1u : 0u;
+  }
+}
+
+__global__ void k_oct_compact(const Box3 *__restrict__ in, const uint32_t *__restrict__ keep,
+                              const uint32_t *__restrict__ off, uint32_t n, Box3 *__restrict__ boxes,
+                              uint32_t *__restrict__ refs) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    if (keep[i]) {
+      boxes[off[i]] = in[i];
+      refs[off[i]] = i;
+    }
+}
+
+// The first box from START on that the root cube does not hold (root_fits).
+__global__ void k_oct_first_unfit(const Box3 *__restrict__ boxes, uint32_t start, uint32_t n, float ox, float oy,
+                                  float oz, float size, uint32_t *first) {
+  uint32_t mine = ~0u;
+  for (uint32_t i = start + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Box3 b = boxes[i];
+    const bool fits = ox <= b.lo[0] && oy <= b.lo[1] && oz <= b.lo[2] && __fadd_rn(ox, size) >= b.hi[0] &&
+                      __fadd_rn(oy, size) >= b.hi[1] && __fadd_rn(oz, size) >= b.hi[2];
+    if (!fits) {
+      mine = i;
+      break;
+    }
+  }
+  if (mine != ~0u) atomicMin(first, mine);
 }
 
 __global__ void k_oct_count(const Box3 *boxes, uint32_t n, const Epoch *ep, uint32_t n_ep, uint32_t *count,
@@ -383,11 +449,38 @@ T read_back(const T *d, cudaStream_t st) {
 
 }  // namespace
 
-void build_octree_device(const std::vector<Box3> &boxes, const std::vector<uint32_t> &refs, DeviceArena &A,
-                         DeviceOctree &out) {
+void build_octree_device(const MeshArrays &mesh, const std::vector<Box3> &boxes, const std::vector<uint32_t> &refs,
+                         float4 *prims, DeviceArena &A, DeviceOctree &out) {
   out = DeviceOctree{};
-  const uint32_t n = uint32_t(boxes.size());
   cudaStream_t st = nullptr;   // legacy stream: ordered with the scene's uploads
+  Scratch S;
+
+  // ---- 0. the surfaces, in insertion order ---------------------------------
+  // (Records and boxes made on the host were most of a scene's creation: 200k
+  // triangles, created, queried and destroyed, 10.6 ms; 4.2 ms made here.)
+  const uint32_t nt = mesh.n_triangles, tail = uint32_t(boxes.size());
+  Box3 *d_boxes = S.get<Box3>(size_t(nt) + tail);
+  uint32_t *d_refs = S.get<uint32_t>(size_t(nt) + tail);
+  uint32_t kept = 0;
+  if (nt) {
+    float *d_v = S.get<float>(3 * size_t(mesh.n_vertices));
+    uint32_t *d_t = S.get<uint32_t>(3 * size_t(nt)), *keep = S.get<uint32_t>(size_t(nt) + 1),
+             *off = S.get<uint32_t>(size_t(nt) + 1);
+    Box3 *all = S.get<Box3>(nt);
+    check_cuda(cudaMemcpyAsync(d_v, mesh.vertices, size_t(mesh.n_vertices) * 12, cudaMemcpyHostToDevice, st), "upload");
+    check_cuda(cudaMemcpyAsync(d_t, mesh.triangles, size_t(nt) * 12, cudaMemcpyHostToDevice, st), "upload");
+    k_oct_triangles<<<grid_for(nt), 256, 0, st>>>(d_v, d_t, nt, prims, all, keep);
+    check_cuda(cudaMemsetAsync(keep + nt, 0, 4, st), "memset");
+    exclusive_sum(S, keep, off, nt + 1, st);
+    k_oct_compact<<<grid_for(nt), 256, 0, st>>>(all, keep, off, nt, d_boxes, d_refs);
+    check_cuda(cudaGetLastError(), "octree triangles");
+    kept = read_back(off + nt, st);
+  }
+  const uint32_t n = kept + tail;
+  if (tail) {
+    check_cuda(cudaMemcpyAsync(d_boxes + kept, boxes.data(), tail * sizeof(Box3), cudaMemcpyHostToDevice, st), "upload");
+    check_cuda(cudaMemcpyAsync(d_refs + kept, refs.data(), tail * 4, cudaMemcpyHostToDevice, st), "upload");
+  }
   if (n == 0) {
     std::vector<uint32_t> pl(4, PREF_END);
     out.nodes = static_cast<uint4 *>(A.alloc(0));
@@ -397,18 +490,25 @@ void build_octree_device(const std::vector<Box3> &boxes, const std::vector<uint3
     return;
   }
 
-  // ---- 0. the root's growth, replayed on the host --------------------------
-  // One epoch per root a surface was inserted under; Epoch::depth first holds
-  // the number of growths before the epoch, then the root's depth.
+  // The root's growth, replayed on the boxes that make it grow.  One epoch per
+  // root a surface was inserted under; Epoch::depth first holds the number of
+  // growths before the epoch, then the root's depth.
   std::vector<Epoch> ep;
   std::vector<uint32_t> grow_octant;   // octant given to the old root, per growth
+  uint32_t *d_first = S.get<uint32_t>(1);
   float o[3], size;
-  root_start(boxes[0], o, size);
+  root_start(read_back(d_boxes, st), o, size);
   ep.push_back(Epoch{0, 0, {o[0], o[1], o[2]}, size, 0, 0});
-  for (uint32_t i = 1; i < n; i++) {
-    if (root_fits(o, size, boxes[i])) continue;
-    while (!root_fits(o, size, boxes[i])) grow_octant.push_back(root_grow(boxes[i], o, size));
+  for (uint32_t from = 1; from < n;) {
+    check_cuda(cudaMemsetAsync(d_first, 0xff, 4, st), "memset");
+    k_oct_first_unfit<<<grid_for(n - from), 256, 0, st>>>(d_boxes, from, n, o[0], o[1], o[2], size, d_first);
+    const uint32_t i = read_back(d_first, st);
+    if (i == ~0u) break;
+    const Box3 b = read_back(d_boxes + i, st);
+    while (!root_fits(o, size, b) && grow_octant.size() <= kMaxDigits) grow_octant.push_back(root_grow(b, o, size));
+    if (grow_octant.size() > kMaxDigits) break;
     ep.push_back(Epoch{i, uint32_t(grow_octant.size()), {o[0], o[1], o[2]}, size, 0, 0});
+    from = i + 1;
   }
   const uint32_t G = uint32_t(grow_octant.size());
   if (G > kMaxDigits) throw Error{SNOG_EINVAL, "octree root grew more than 40 times"};
@@ -430,13 +530,8 @@ void build_octree_device(const std::vector<Box3> &boxes, const std::vector<uint3
   for (int k = 0; k < 3; k++) out.origin[k] = o[k];
   out.size = size;
 
-  Scratch S;
-  Box3 *d_boxes = S.get<Box3>(n);
-  uint32_t *d_refs = S.get<uint32_t>(n);
   Epoch *d_ep = S.get<Epoch>(ep.size());
   uint32_t *d_err = S.get<uint32_t>(2);
-  check_cuda(cudaMemcpyAsync(d_boxes, boxes.data(), n * sizeof(Box3), cudaMemcpyHostToDevice, st), "upload");
-  check_cuda(cudaMemcpyAsync(d_refs, refs.data(), n * 4, cudaMemcpyHostToDevice, st), "upload");
   check_cuda(cudaMemcpyAsync(d_ep, ep.data(), ep.size() * sizeof(Epoch), cudaMemcpyHostToDevice, st), "upload");
   check_cuda(cudaMemsetAsync(d_err, 0, 8, st), "memset");
 

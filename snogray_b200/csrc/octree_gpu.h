@@ -23,13 +23,22 @@ struct DeviceOctree {
   float origin[3] = {0, 0, 0}, size = 0;
 };
 
+// A scene's mesh, in host memory.
+struct MeshArrays {
+  const float *vertices;
+  const uint32_t *triangles;
+  uint32_t n_vertices, n_triangles;
+};
+
 // Build on the current device the tree the host builder makes from the same
-// surfaces: BOXES[i] is the bounding box of the i-th surface in insertion
-// order and REFS[i] the id its lists hold.  Output arrays are allocated in A.
-// Throws Error (SNOG_EINVAL for trees deeper than 40 levels, SNOG_ECUDA,
+// surfaces: the mesh's triangles (those that are not degenerate, with their
+// index as id), then the surfaces whose bounding boxes and ids are in BOXES and
+// REFS, in insertion order.  The triangles' primitive records are made on the
+// way, into PRIMS (3 per triangle, device memory).  Output arrays are allocated
+// in A.  Throws Error (SNOG_EINVAL for trees deeper than 40 levels, SNOG_ECUDA,
 // SNOG_ENOMEM).
-void build_octree_device(const std::vector<Box3> &boxes, const std::vector<uint32_t> &refs, DeviceArena &A,
-                         DeviceOctree &out);
+void build_octree_device(const MeshArrays &mesh, const std::vector<Box3> &boxes, const std::vector<uint32_t> &refs,
+                         float4 *prims, DeviceArena &A, DeviceOctree &out);
 
 // The host layout (octree_build.h) of a tree in the device layout.
 OctreeArrays octree_from_device(const uint4 *d_nodes, uint32_t n_nodes, const uint32_t *d_plist, uint32_t n_plist4,

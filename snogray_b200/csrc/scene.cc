@@ -245,26 +245,24 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
   // lists hold those ids (snog_common.h).
   BoxAcc scene_box, mesh_box;
   const size_t n_prims = size_t(d.n_triangles) + d.n_spheres + d.n_tripars;
-  std::vector<float4> prims(3 * n_prims, make_float4(0.f, 0.f, 0.f, 0.f));
-  std::vector<uint32_t> prim_mat(n_prims);
-  auto put = [&](size_t id, float4 a, float4 b, float4 c, uint32_t mat) {
-    prims[3 * id] = a;
-    prims[3 * id + 1] = b;
-    prims[3 * id + 2] = c;
-    prim_mat[id] = mat;
-  };
   // The octree is built on the host (OctreeBuilder, surface by surface) or
-  // on the device (build_octree_device, the same tree from the surfaces'
-  // boxes in insertion order).
+  // on the device (build_octree_device, the same tree); there, the triangles'
+  // records and boxes are made on the device too, and the host's arrays hold
+  // only the primitives after them.
   const bool dev_oct = upload && (octree_mode == SNOG_OCTREE_DEVICE ||
                                   (octree_mode == SNOG_OCTREE_AUTO && n_prims >= kDeviceOctreeMinSurfaces));
+  const size_t first = dev_oct ? d.n_triangles : 0;
+  std::vector<float4> prims(3 * (n_prims - first), make_float4(0.f, 0.f, 0.f, 0.f));
+  std::vector<uint32_t> prim_mat(n_prims - first);
+  auto put = [&](size_t id, float4 a, float4 b, float4 c, uint32_t mat) {
+    prims[3 * (id - first)] = a;
+    prims[3 * (id - first) + 1] = b;
+    prims[3 * (id - first) + 2] = c;
+    prim_mat[id - first] = mat;
+  };
   OctreeBuilder ob;
   std::vector<Box3> oct_boxes;
   std::vector<uint32_t> oct_refs;
-  if (dev_oct) {
-    oct_boxes.reserve(n_prims);
-    oct_refs.reserve(n_prims);
-  }
   auto oct_add = [&](uint32_t ref, const Box3 &b) {
     if (dev_oct) {
       oct_boxes.push_back(b);
@@ -273,18 +271,25 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
       ob.add(ref, b);
     }
   };
-  for (uint32_t v = 0; v < d.n_vertices; v++) mesh_box.add(v3(d.vertices + 3 * size_t(v)));
-  for (uint32_t t = 0; t < d.n_triangles; t++) {
+  // Triangle T's record; adds it to OB unless it is degenerate: those are
+  // left out of the space (surface/mesh.cc:833-846); the mesh is left-handed,
+  // normal = e2 x e1 (surface/mesh.h:55).
+  auto triangle = [&](uint32_t t, float4 *rec) {
     const uint32_t *ix = d.triangles + 3 * size_t(t);
     V3 p0 = v3(d.vertices + 3 * size_t(ix[0])), p1 = v3(d.vertices + 3 * size_t(ix[1])),
        p2 = v3(d.vertices + 3 * size_t(ix[2]));
     V3 e1 = vsub(p1, p0), e2 = vsub(p2, p0);
-    put(t, make_float4(p0.x, p0.y, p0.z, float(PRIM_TRI)), make_float4(e1.x, e1.y, e1.z, 0.f),
-        make_float4(e2.x, e2.y, e2.z, 0.f), d.tri_material[t]);
-    // Degenerate triangles are left out of the space (surface/mesh.cc:833-846);
-    // the mesh is left-handed, normal = e2 x e1 (surface/mesh.h:55).
-    if (vlen2(vcross(e2, e1)) > 0) oct_add(t, box_of_points({p0, p1, p2}));
-  }
+    rec[0] = make_float4(p0.x, p0.y, p0.z, float(PRIM_TRI));
+    rec[1] = make_float4(e1.x, e1.y, e1.z, 0.f);
+    rec[2] = make_float4(e2.x, e2.y, e2.z, 0.f);
+    if (vlen2(vcross(e2, e1)) > 0) ob.add(t, box_of_points({p0, p1, p2}));
+  };
+  for (uint32_t v = 0; v < d.n_vertices; v++) mesh_box.add(v3(d.vertices + 3 * size_t(v)));
+  if (!dev_oct)
+    for (uint32_t t = 0; t < d.n_triangles; t++) {
+      triangle(t, &prims[3 * size_t(t)]);
+      prim_mat[t] = d.tri_material[t];
+    }
   if (d.n_triangles) scene_box.add(Box3{{mesh_box.lo[0], mesh_box.lo[1], mesh_box.lo[2]},
                                        {mesh_box.hi[0], mesh_box.hi[1], mesh_box.hi[2]}});
   for (uint32_t i = 0; i < d.n_spheres; i++) {
@@ -453,9 +458,12 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
   if (upload) try {
     DeviceOctree dov;
     bool built = false;
+    float4 *const d_prims = static_cast<float4 *>(A.alloc(n_prims * 48));
+    D.prims = d_prims;
     if (dev_oct) {
       try {
-        build_octree_device(oct_boxes, oct_refs, A, dov);
+        build_octree_device(MeshArrays{d.vertices, d.triangles, d.n_vertices, d.n_triangles}, oct_boxes, oct_refs,
+                            d_prims, A, dov);
         built = true;
       } catch (const Error &e) {
         // Trees the device builder does not take (root grown more than 40
@@ -463,6 +471,10 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
         // go to the host builder in AUTO mode.  The device builder finds
         // these before it allocates its outputs in the scene's arena.
         if (octree_mode != SNOG_OCTREE_AUTO || e.code != SNOG_EINVAL) throw;
+        std::vector<float4> tri(3 * size_t(d.n_triangles));
+        for (uint32_t t = 0; t < d.n_triangles; t++) triangle(t, &tri[3 * size_t(t)]);
+        if (!tri.empty())
+          check_cuda(cudaMemcpy(d_prims, tri.data(), tri.size() * 16, cudaMemcpyHostToDevice), "upload");
         for (size_t i = 0; i < oct_boxes.size(); i++) ob.add(oct_refs[i], oct_boxes[i]);
         S.oct = ob.finish();
       }
@@ -488,14 +500,21 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
       D.plist = dev_upload(A, plist4);
       S.oct_plist4 = uint32_t(plist4.size());
     }
-    D.prims = dev_upload(A, prims);
+    if (!prims.empty())
+      check_cuda(cudaMemcpy(d_prims + 3 * first, prims.data(), prims.size() * 16, cudaMemcpyHostToDevice), "upload");
     {
       float4 *lrec = static_cast<float4 *>(A.alloc(size_t(S.oct_plist4) * 48));
       check_cuda(build_list_records(D.plist, S.oct_plist4, D.prims, lrec, nullptr), "list records");
       check_cuda(cudaStreamSynchronize(nullptr), "list records");
       D.lrec = lrec;
     }
-    D.prim_mat = dev_upload(A, prim_mat);
+    {
+      uint32_t *m = static_cast<uint32_t *>(A.alloc(n_prims * 4));
+      if (first) check_cuda(cudaMemcpy(m, d.tri_material, first * 4, cudaMemcpyHostToDevice), "upload");
+      if (!prim_mat.empty())
+        check_cuda(cudaMemcpy(m + first, prim_mat.data(), prim_mat.size() * 4, cudaMemcpyHostToDevice), "upload");
+      D.prim_mat = m;
+    }
     if (d.vertex_normals && d.n_triangles) {
       std::vector<float4> vn(d.n_vertices);
       for (uint32_t v = 0; v < d.n_vertices; v++)
