@@ -79,8 +79,9 @@ __device__ __forceinline__ bool tripar_hit(float3 corner, float3 e1, float3 e2, 
 
 // tripar_hit evaluated to the end without early exits: the same
 // operations and the same result, but a warp whose lanes would leave at
-// different tests does not diverge.  Measured faster where rounds are full
-// of long lists (the intersection batch, +2.4 %), not on any-hit rounds.
+// different tests does not diverge.  What list rounds use (against early exits:
+// the intersection batch +2.4 %; shadow rays of the terrain frame 51.2 -> 50.7
+// ms, of a Cornell render 0.653 -> 0.626).
 __device__ __forceinline__ bool tripar_hit_flat(float3 corner, float3 e1, float3 e2, bool parallelogram,
                                                 float3 o, float3 d, float t0, float t1, float &t) {
   const float3 pvec = xcross(d, e2);
@@ -170,22 +171,13 @@ __device__ __forceinline__ PrimRec load_prim(const DevScene &s, uint32_t id) {
 // Test a loaded primitive against the ray; closest queries shrink t1 on a
 // hit (the surface's intersect / intersects methods, surface/mesh.cc:730-760,
 // surface/sphere.cc:110-125, surface/tripar.cc:93-115).
-// FLAT: triangles and tripars through tripar_hit_flat.
-template <bool FLAT = false>
 __device__ __forceinline__ bool test_prim(const PrimRec &r, float3 o, float3 d, float t0, float &t1) {
   const float kind = r.a.w;
-  float t, u, v;
-  if (kind == float(PRIM_SPHERE)) {
-    if (sphere_hit(xyz(r.a), r.b.x, o, d, t0, t1, t)) {
-      t1 = t;
-      return true;
-    }
-    return false;
-  }
-  const bool hit = FLAT ? tripar_hit_flat(xyz(r.a), xyz(r.b), xyz(r.c), kind == float(PRIM_PARALLELOGRAM), o, d,
-                                          t0, t1, t)
-                       : tripar_hit(xyz(r.a), xyz(r.b), xyz(r.c), kind == float(PRIM_PARALLELOGRAM), o, d, t0, t1,
-                                    t, u, v);
+  float t;
+  const bool hit = kind == float(PRIM_SPHERE)
+                       ? sphere_hit(xyz(r.a), r.b.x, o, d, t0, t1, t)
+                       : tripar_hit_flat(xyz(r.a), xyz(r.b), xyz(r.c), kind == float(PRIM_PARALLELOGRAM), o, d, t0,
+                                         t1, t);
   if (hit) t1 = t;
   return hit;
 }
@@ -615,12 +607,12 @@ __device__ __forceinline__ bool list_round(Traversal<STACK> &tr, bool any, Trace
     const float4 *p = reinterpret_cast<const float4 *>(o_lrec) + 3 * size_t(unit.x + kPer * lane);
     const PrimRec r0{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
     th = rt1;
-    hit = test_prim<ANY != kAnyOnly>(r0, ro, rd, rt0, th);
+    hit = test_prim(r0, ro, rd, rt0, th);
     pid = __float_as_uint(r0.c.w);
     if (kPer == 2u && kPer * lane + 1u < (unit.y >> 8) && !(ANY != kClosestOnly && hit && (unit.y & 32u))) {
       const PrimRec r1{__ldg(p + 3), __ldg(p + 4), __ldg(p + 5)};
       float th1 = rt1;
-      const bool hit1 = test_prim<ANY != kAnyOnly>(r1, ro, rd, rt0, th1);
+      const bool hit1 = test_prim(r1, ro, rd, rt0, th1);
       // The later entry wins only with a smaller t (the earlier one keeps ties).
       if (hit1 && (!hit || th1 < th)) {
         hit = true;
