@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "launch.h"
@@ -21,7 +22,7 @@ namespace snog {
 // 16M rays in 1M triangles 16.4 ms at 7 blocks, 15.7 at 8.
 constexpr int batch_blocks(bool count) { return count ? 7 : 8; }
 
-template <int STACK, bool COUNT>
+template <int STACK, int PER, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, batch_blocks(COUNT)) k_trace_batch(DevScene s, const float *__restrict__ rays,
                                                      uint32_t n, uint32_t n_closest,
                                                      int32_t *__restrict__ prim, float *__restrict__ tout,
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(kTraceBlock, batch_blocks(COUNT)) k_trace_batc
       at += c.tests - base.tests;
     }
   };
-  trace_loop<STACK, kMixed, 2, COUNT>(fetch, n, c, start, done);
+  trace_loop<STACK, kMixed, PER, COUNT>(fetch, n, c, start, done);
   if (c.overflow) atomicOr(err, 1u);
   if (COUNT) {
     // All lanes reach this point: reduce per warp, one atomic per warp.
@@ -178,16 +179,27 @@ cudaError_t launch_trace_batch(const DevScene &s, const float *rays, uint32_t n,
   // A warp per ray while the resident grid has them: a small batch takes as
   // long as its slowest warp (RayDispenser).
   const uint32_t want = n / (threads / 32) + (n % (threads / 32) ? 1u : 0u);
-  auto launch = [&](auto kernel) {
+  auto launch = [&](auto stack) {
+    // List entries are dealt in pairs where lists along rays are long and the
+    // launch fills every lane: a fuller round costs less per entry, but warps
+    // with a few rays wait for the longer rounds.  Pairs / single entries, 2M
+    // closest-hit rays in scenes of 0.7, 1.4, 1.8, 3.6, 5.4 and 9 tests per node
+    // visit: 2.25 / 1.87 ms, 1.02 / 0.92, 2.22 / 2.18, 2.31 / 2.42, 1.71 / 1.86,
+    // 3.16 / 3.46; at 5.4, 300k rays 0.347 / 0.370 ms, 30k 0.142 / 0.130, 1000
+    // 0.084 / 0.075.
+    constexpr int kStack = stack();
+    const bool pairs = s.pair_lists && n >= uint32_t(num_sms()) * batch_blocks(false) * kTraceBlock;
+    const auto kernel = counters ? (pairs ? k_trace_batch<kStack, 2, true> : k_trace_batch<kStack, 1, true>)
+                                 : (pairs ? k_trace_batch<kStack, 2, false> : k_trace_batch<kStack, 1, false>);
     const uint32_t resident = resident_grid(kernel, threads);
     kernel<<<want < resident ? want : resident, threads, 0, st>>>(s, rays, n, n_closest, prim, t, nrm, counters, err,
                                                                   fetch);
   };
   switch (stack_class_for_depth(s.max_depth)) {
-    case 32: counters ? launch(k_trace_batch<32, true>) : launch(k_trace_batch<32, false>); break;
-    case 64: counters ? launch(k_trace_batch<64, true>) : launch(k_trace_batch<64, false>); break;
-    case 128: counters ? launch(k_trace_batch<128, true>) : launch(k_trace_batch<128, false>); break;
-    case 256: counters ? launch(k_trace_batch<256, true>) : launch(k_trace_batch<256, false>); break;
+    case 32: launch(std::integral_constant<int, 32>{}); break;
+    case 64: launch(std::integral_constant<int, 64>{}); break;
+    case 128: launch(std::integral_constant<int, 128>{}); break;
+    case 256: launch(std::integral_constant<int, 256>{}); break;
     default: return cudaErrorInvalidValue;
   }
   if (launches) (*launches)++;

@@ -48,3 +48,25 @@ def test_long_lists_with_ties(n, n_rays):
         hit = np.nonzero(prim[:nc] >= 0)[0]
         assert np.array_equal(t[hit].view(np.uint32), ref_t[hit].view(np.uint32))
         assert cnt["closest_tests"] == ref["closest"]["surface_tests"]   # one node: every entry once
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fill", [-1, 0])
+def test_batches_around_a_full_device(fill):
+    """Long lists along rays, one ray fewer than the device's trace lanes (8
+    blocks of 128 per SM) and as many: entries dealt singly and in pairs."""
+    import torch
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 8 * 128 + fill
+    sd = scenes.random_triangles(5000, seed=4, edge_lo=0.02, edge_hi=0.1)
+    rays = scenes.random_rays(n, seed=6)
+    nc = n // 2
+    ref_prim, ref_t, _, _, _ = spec.port_trace(sd, rays, nc, threads=8)
+    with Scene(sd) as sc:
+        assert sc.info()["pair_lists"] == 1
+        prim, t, _, _ = sc.trace(rays, nc)
+        dev = torch.empty(n, dtype=torch.int32, device="cuda")
+        sc.trace_device(torch.from_numpy(rays).cuda().data_ptr(), n, nc, dev.data_ptr())
+        torch.cuda.synchronize()
+    assert np.array_equal(prim, ref_prim) and np.array_equal(dev.cpu().numpy(), ref_prim)
+    hit = np.nonzero(prim[:nc] >= 0)[0]
+    assert np.array_equal(t[hit].view(np.uint32), ref_t[hit].view(np.uint32))
