@@ -35,6 +35,14 @@ uint32_t resident_grid(K kernel, int threads) {
 cudaError_t build_list_records(const uint32_t *plist, uint32_t n, const float4 *prims, float4 *lrec,
                                cudaStream_t st);
 
+// Fill GUIDE, CELLS + 2 entries for each of the ROWS cumulative distributions of N
+// values at CDF: entry b the first value at or above b / CELLS, the last N.  The
+// first value at or above v, 0 <= v <= 1, then lies between the entries of v's
+// cell and the next.  CELLS: a power of two, so that a value's cell is exact, or 0
+// for values that do not ascend, which are searched whole.
+cudaError_t build_cdf_guide(const float *cdf, uint32_t n, uint32_t rows, uint32_t cells, uint32_t *guide,
+                            cudaStream_t st);
+
 // Whether the closest-hit kernels should deal list entries in pairs for
 // scene S: traces 8192 random rays through its bounding box and answers yes
 // when they test more than 2.5 primitives per node visit (long lists along

@@ -379,6 +379,7 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
   std::vector<float4> texels;
   std::vector<float> row_cdf, col_cdf;
   uint32_t lw = 0, lh = 0;
+  bool ascending = true;   // each cumulative distribution, from 0 on
   if (d.env_width) {
     DevLight L{};
     L.type = LS_ENV;
@@ -429,6 +430,7 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
     for (uint32_t row = 0; row < lh; row++) {
       for (uint32_t col = 0; col < lw; col++) norm_sum += double(bins[size_t(row) * lw + col]) * inv_bin_sum;
       row_cdf[row] = float(norm_sum);
+      ascending = ascending && row_cdf[row] >= (row ? row_cdf[row - 1] : 0.f);
     }
     for (uint32_t row = 0; row < lh; row++) {
       double row_sum = 0;
@@ -437,7 +439,9 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
       double acc = 0;
       for (uint32_t col = 0; col < lw; col++) {
         acc += double(bins[size_t(row) * lw + col]) * inv_row_sum;
-        col_cdf[size_t(row) * lw + col] = float(acc);
+        float *c = &col_cdf[size_t(row) * lw + col];
+        *c = float(acc);
+        ascending = ascending && *c >= (col ? c[-1] : 0.f);
       }
     }
   }
@@ -532,6 +536,18 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
     D.env_texels = dev_upload(A, texels);
     D.env_row_cdf = dev_upload(A, row_cdf);
     D.env_col_cdf = dev_upload(A, col_cdf);
+    if (lw) {
+      auto guide = [&](const float *cdf, uint32_t n, uint32_t rows, uint32_t &cells) {
+        cells = ascending ? 1u : 0u;
+        while (cells && cells < n) cells *= 2u;
+        uint32_t *g = static_cast<uint32_t *>(A.alloc(size_t(rows) * (size_t(cells) + 2) * 4));
+        check_cuda(build_cdf_guide(cdf, n, rows, cells, g, nullptr), "light map guide");
+        return g;
+      };
+      D.env_row_guide = guide(D.env_row_cdf, lh, 1, D.row_cells);
+      D.env_col_guide = guide(D.env_col_cdf, lw, lh, D.col_cells);
+      check_cuda(cudaStreamSynchronize(nullptr), "light map guide");
+    }
   } catch (...) {
     device_idle(S.device);
     A.release();

@@ -115,9 +115,11 @@ struct DevScene {
   const float4 *env_texels;   // env_w * env_h, row 0 = top image row
   const float *env_row_cdf;   // lmap_h
   const float *env_col_cdf;   // lmap_w * lmap_h
+  const uint32_t *env_row_guide, *env_col_guide;   // where to search these (build_cdf_guide)
   uint32_t n_nodes, n_tri, n_sph, n_tpar;
   uint32_t n_mats, n_lights, n_media, env_light;   // env_light: light index or ~0u
   uint32_t env_w, env_h, lmap_w, lmap_h;
+  uint32_t row_cells, col_cells;   // cells of the guides: powers of two, or 0
   float env_frame[9];
   float origin[3], size;      // octree root cube
   float bbox_min[3], bbox_max[3];

@@ -690,7 +690,23 @@ void launch_bounce(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, uint
   if (prof) prof->end(st);
 }
 
+__global__ void k_cdf_guide(const float *cdf, uint32_t n, uint32_t rows, uint32_t cells, uint32_t *guide) {
+  const uint64_t width = uint64_t(cells) + 2u;
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < rows * width;
+       i += uint64_t(gridDim.x) * blockDim.x) {
+    const uint64_t row = i / width;
+    const uint32_t b = uint32_t(i % width);
+    guide[i] = b == 0u ? 0u : b > cells ? n : lower_bound_f(cdf + row * n, 0u, n, float(b) / float(cells));
+  }
+}
+
 }  // namespace
+
+cudaError_t build_cdf_guide(const float *cdf, uint32_t n, uint32_t rows, uint32_t cells, uint32_t *guide,
+                            cudaStream_t st) {
+  k_cdf_guide<<<uint32_t(num_sms()) * 8, 256, 0, st>>>(cdf, n, rows, cells, guide);
+  return cudaGetLastError();
+}
 
 cudaError_t RenderProfile::begin(cudaStream_t st, int kind) {
   if (n == cap) {
