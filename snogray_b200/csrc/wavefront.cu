@@ -24,7 +24,7 @@
 //
 // Path state is SoA of 16-byte records (float4 throughput+rr ratio, float4
 // radiance+alpha) plus a 32-bit word: path length (8 bits), after-specular
-// (1 bit), media-stack depth (2 bits) and up to three medium ids (7 bits
+// (1 bit), media-stack depth (3 bits) and up to four medium ids (5 bits
 // each).  Queues hold rays as two float4 (origin+t0, direction+t1) in queue
 // order, so the trace kernels read them with coalesced 128-bit loads.
 
