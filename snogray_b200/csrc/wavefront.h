@@ -96,18 +96,18 @@ struct RenderProfile {
   ~RenderProfile();
 };
 
-// Render a whole job on STREAM into accum (float4 colour*weight sums + float
-// weight, W*H each; zeroed here) and resolve it to out_rgb (W*H*3 floats,
-// device).  Paths are processed in waves of at most wb.wave_cap.  With PROF,
-// every launch is bracketed by events; with COUNT (or PROF) the traversal
-// counts its node visits and primitive tests into wb.stats[2..5].  With SIDE
-// (and no PROF) shadow rays run beside the next bounce's closest hits.
 // Mitchell-filter all TOTAL samples of a finished job (radiance + alpha and
 // camera jitter per path, pattern-pixel-major) into its image: clears
 // accum/wsum, gathers, resolves into out_rgb.
 cudaError_t splat_job(const JobConsts &jc, const float4 *rad, const float2 *jit, uint64_t total, float4 *accum,
                       float *wsum, float *out_rgb, cudaStream_t st);
 
+// Render a whole job on STREAM into accum (float4 colour*weight sums + float
+// weight, W*H each; zeroed here) and resolve it to out_rgb (W*H*3 floats,
+// device).  Paths are processed in waves of at most wb.wave_cap.  With PROF,
+// every launch is bracketed by events; with COUNT (or PROF) the traversal
+// counts its node visits and primitive tests into wb.stats[2..5].  With SIDE
+// (and no PROF) shadow rays run beside the next bounce's closest hits.
 cudaError_t render_job(const DevScene &s, const JobConsts &jc, WaveBuffers &wb, float4 *accum,
                        float *wsum, float *out_rgb, cudaStream_t st, uint32_t *waves, uint32_t *launches,
                        RenderProfile *prof = nullptr, bool count = false, ShadowStream *side = nullptr);
