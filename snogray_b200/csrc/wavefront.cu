@@ -28,6 +28,7 @@
 // each).  Queues hold rays as two float4 (origin+t0, direction+t1) in queue
 // order, so the trace kernels read them with coalesced 128-bit loads.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -38,6 +39,8 @@
 #include "pathstate.cuh"
 #include "scene.h"
 #include "wavefront.h"
+
+namespace cg = cooperative_groups;
 
 namespace snog {
 
@@ -485,9 +488,35 @@ __device__ __forceinline__ float mitchell1(float x) {
   return x > 2.f ? 0.f : x > 1.f ? outer : inner;
 }
 
-// Target pixels of a splat block: a thread takes kSplatRows of one column.
-constexpr int kSplatW = 32, kSplatRows = 4, kSplatWarps = 4, kSplatH = kSplatRows * kSplatWarps;
-constexpr int kHaloW = kSplatW + 4, kHaloH = kSplatH + 4, kHalo = kHaloW * kHaloH;
+// A splat block's target pixels -- a thread takes ROWS of one column -- and the
+// pattern pixels around them.
+constexpr int kSplatW = 32, kSplatWarps = 4, kSplatBlock = 32 * kSplatWarps, kHaloW = kSplatW + 4;
+constexpr uint32_t kSplatSplit = 16;   // most blocks per tile
+constexpr int splat_height(int rows) { return rows * kSplatWarps; }
+constexpr int splat_tile(int rows) { return kSplatW * splat_height(rows); }
+constexpr int splat_halo(int rows) { return kHaloW * (splat_height(rows) + 4); }
+
+// What a splat block keeps of one sample of each pattern pixel around its tile.
+template <int ROWS>
+struct SplatSlice {
+  float4 col[splat_halo(ROWS)];   // alpha-scaled colour, alpha
+  float wlo[splat_halo(ROWS)];    // the least weight the clamp lets pass
+  // [d]: weight for the target d - 2 pixels to the left / above
+  float wx[5][splat_halo(ROWS)], wy[5][splat_halo(ROWS)];
+};
+
+// Its sums (colour, alpha, weight), for the other blocks of its tile.
+template <int ROWS>
+struct SplatSums {
+  double v[5][splat_tile(ROWS)];
+};
+
+template <int ROWS>
+union SplatShared {
+  SplatSlice<ROWS> slice;
+  SplatSums<ROWS> sums;
+  __device__ SplatShared() {}
+};
 
 // Gather the wave's samples into the target pixels they reach
 // (ImageFilterConv::add_sample, image/image-filter-conv.h:109-186): every
@@ -496,45 +525,43 @@ constexpr int kHaloW = kSplatW + 4, kHaloH = kSplatH + 4, kHalo = kHaloW * kHalo
 //
 // Every sample reaches 25 pixels, so what a pixel and a sample cost together
 // is what counts.  A block takes one sample of each pattern pixel around its
-// 32x16 targets at a time: first each sample's colour, its five weights per
-// axis and its clamp go to shared memory, then every thread adds the products
-// for its four targets -- two products, five fused additions and no branch
-// each, with a sample's colour read once for up to four targets.  The clamp
+// 32x16 targets (32x4 in small images) at a time: first each sample's colour, its
+// five weights per axis and its clamp go to shared memory, then every thread adds
+// the products for its four targets (one) -- two products, five fused additions
+// and no branch each, with a sample's colour read once for up to four.  The clamp
 // scales a product whose smallest component lies below -0.1 to it, which is
 // to say that the weight is at least -0.1 / largest component.
-// The blocks of one tile take every gridDim.x-th sample each; with more than
-// one, the sums meet in atomic additions, so small images at many samples fill
-// the device too, and the tile's blocks run together, so that what one of them
-// leaves of a memory sector is still in L2 for the next.
-// (Bound by shared-memory latency at 20 warps per SM.  Against lanes that each
-// evaluated the filter for every pair of sample and target: 853x479 pixels at 9
-// samples 817 -> 145 us, 256x256 at 16 136 -> 53 us, at 64 510 -> 176 us.  Two
-// or one target per thread in more warps: 253 and 184 us on the first.)
-template <bool ATOMIC>
-__global__ void __launch_bounds__(32 * kSplatWarps, 5) k_splat(JobConsts jc, uint64_t base, uint32_t n,
+//
+// A slice's 25 products per target are summed in 32 bits, and the slices in 64:
+// all products in one 32-bit sum round worse by the square root of the samples
+// (rms of a pixel 3.2e-7 at 16 samples, 6e-7 at 64; 6e-8 so).  The blocks of one
+// tile are a cluster and take every gridDim.x-th sample each; their sums are
+// added in the order of the blocks, so that an image repeats bit for bit.
+// (Bound by shared-memory latency at 16 warps per SM; at 20 the 64-bit sums do not
+// fit the registers: 1920x1080 at 16 samples 1.64 ms, 2.75 at 20 warps.  Against
+// lanes that each evaluated the filter for every pair of sample and target, with
+// k_camera and k_resolve: 853x479 pixels at 9 samples 876 -> 208 us, 256x256 at 16
+// 162 -> 81, at 64 579 -> 235.  Two or one target per thread in more warps:
+// slower by half and by a quarter.)
+template <int ROWS, bool CLUSTER>
+__global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t base, uint32_t n,
                                                           const float4 *__restrict__ rad,
                                                           const float2 *__restrict__ jit, float4 *accum, float *wsum,
                                                           int ty0, int nrows) {
   start_after_previous();
-  __shared__ float4 col[kHalo];                  // alpha-scaled colour, alpha
-  __shared__ float wlo[kHalo];                   // the least weight the clamp lets pass
-  __shared__ float wx[5][kHalo], wy[5][kHalo];   // [d]: weight for the target d - 2 pixels to the left / above
+  constexpr int kHalo = splat_halo(ROWS), kTile = splat_tile(ROWS);
+  __shared__ SplatShared<ROWS> shared;
+  SplatSlice<ROWS> &sl = shared.slice;
   const uint32_t p0 = uint32_t(base / jc.S), p1 = uint32_t((base + n) / jc.S);
   const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
-  const int x0 = int(blockIdx.y) * kSplatW, y0 = ty0 + int(blockIdx.z) * kSplatH;
-  float4 acc[kSplatRows];
-  float wacc[kSplatRows];
-#pragma unroll
-  for (int r = 0; r < kSplatRows; r++) {
-    acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-    wacc[r] = 0.f;
-  }
+  const int x0 = int(blockIdx.y) * kSplatW, y0 = ty0 + int(blockIdx.z) * splat_height(ROWS);
+  double sum[ROWS][5] = {};   // colour, alpha, weight
   // This thread's pattern pixels around the tile, from the wave's first on.
-  constexpr int kRounds = (kHalo + 32 * kSplatWarps - 1) / (32 * kSplatWarps);
+  constexpr int kRounds = (kHalo + kSplatBlock - 1) / kSplatBlock;
   uint32_t pix[kRounds];
 #pragma unroll
   for (int q = 0; q < kRounds; q++) {
-    const int i = int(threadIdx.x) + q * 32 * kSplatWarps;
+    const int i = int(threadIdx.x) + q * kSplatBlock;
     const int pc = jc.OX + x0 - 2 + i % kHaloW - jc.PX, pr = jc.OY + y0 - 2 + i / kHaloW - jc.PY;
     const uint32_t pidx = uint32_t(pr) * jc.PW + uint32_t(pc);
     const bool in = i < kHalo && pc >= 0 && pc < int(jc.PW) && pr >= 0 && pr < int(jc.PH) && pidx >= p0 && pidx < p1;
@@ -557,35 +584,42 @@ __global__ void __launch_bounds__(32 * kSplatWarps, 5) k_splat(JobConsts jc, uin
     }
 #pragma unroll
     for (int q = 0; q < kRounds; q++) {
-      const int i = int(threadIdx.x) + q * 32 * kSplatWarps;
+      const int i = int(threadIdx.x) + q * kSplatBlock;
       if (i >= kHalo) break;
       const float4 r = rq[q];
       // Tint (radiance, alpha) stores alpha-scaled colour (color/tint.h:45-49)
       const float4 c = make_float4(r.x * r.w, r.y * r.w, r.z * r.w, r.w);
-      col[i] = c;
-      wlo[i] = -0.1f / fmaxf(fmaxf(c.x, fmaxf(c.y, c.z)), 0.f);   // (-inf where nothing is positive)
+      sl.col[i] = c;
+      sl.wlo[i] = -0.1f / fmaxf(fmaxf(c.x, fmaxf(c.y, c.z)), 0.f);   // (-inf where nothing is positive)
       wild |= !(fabsf(c.x) < INFINITY && fabsf(c.y) < INFINITY && fabsf(c.z) < INFINITY && fabsf(c.w) < INFINITY);
       const int px = jc.OX + x0 - 2 + i % kHaloW, py = jc.OY + y0 - 2 + i / kHaloW;
       const float sx = float(px) + jq[q].x, sy = float(py) + jq[q].y;
 #pragma unroll
       for (int d = 0; d < 5; d++) {
-        wx[d][i] = pix[q] != ~0u ? mitchell1(sx - (float(px - (d - 2)) + 0.5f)) : 0.f;
-        wy[d][i] = mitchell1(sy - (float(py - (d - 2)) + 0.5f));
+        sl.wx[d][i] = pix[q] != ~0u ? mitchell1(sx - (float(px - (d - 2)) + 0.5f)) : 0.f;
+        sl.wy[d][i] = mitchell1(sy - (float(py - (d - 2)) + 0.5f));
       }
+    }
+    float4 acc[ROWS];
+    float wacc[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      wacc[r] = 0.f;
     }
     // A zero weight is skipped where an infinite colour could meet it.
     auto add = [&](auto guard) {
 #pragma unroll 1
       for (int dx = 0; dx < 5; dx++) {
 #pragma unroll
-        for (int h = 0; h < kSplatRows + 4; h++) {
-          const int i = (group * kSplatRows + h) * kHaloW + lane + dx;
-          const float4 c = col[i];
-          const float ux = wx[dx][i], lo = wlo[i];
+        for (int h = 0; h < ROWS + 4; h++) {
+          const int i = (group * ROWS + h) * kHaloW + lane + dx;
+          const float4 c = sl.col[i];
+          const float ux = sl.wx[dx][i], lo = sl.wlo[i];
 #pragma unroll
-          for (int r = 0; r < kSplatRows; r++) {
+          for (int r = 0; r < ROWS; r++) {
             if (h < r || h > r + 4) continue;
-            const float w = fmaxf(ux * wy[h - r][i], lo);
+            const float w = fmaxf(ux * sl.wy[h - r][i], lo);
             if (guard() && w == 0.f) continue;
             acc[r].x = fmaf(c.x, w, acc[r].x);
             acc[r].y = fmaf(c.y, w, acc[r].y);
@@ -598,42 +632,89 @@ __global__ void __launch_bounds__(32 * kSplatWarps, 5) k_splat(JobConsts jc, uin
     };
     if (__syncthreads_or(wild)) add(std::true_type{});
     else add(std::false_type{});
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      sum[r][0] += acc[r].x;
+      sum[r][1] += acc[r].y;
+      sum[r][2] += acc[r].z;
+      sum[r][3] += acc[r].w;
+      sum[r][4] += wacc[r];
+    }
     __syncthreads();
   }
-  const int tx = x0 + lane;
-  if (tx >= int(jc.W)) return;
+  auto store = [&](int i, const double *v) {   // add V to target I of the tile
+    const int x = x0 + i % kSplatW, y = y0 + i / kSplatW;
+    if (x >= int(jc.W) || y >= ty0 + nrows) return;
+    const size_t o = size_t(y) * jc.W + size_t(x);
+    const float4 a = accum[o];
+    accum[o] = make_float4(a.x + float(v[0]), a.y + float(v[1]), a.z + float(v[2]), a.w + float(v[3]));
+    wsum[o] += float(v[4]);
+  };
+  if (!CLUSTER) {
 #pragma unroll
-  for (int r = 0; r < kSplatRows; r++) {
-    const int ty = y0 + group * kSplatRows + r;
-    if (ty >= ty0 + nrows) break;
-    const size_t o = size_t(ty) * jc.W + size_t(tx);
-    if (ATOMIC) {
-      float *a = reinterpret_cast<float *>(accum + o);
-      atomicAdd(a, acc[r].x);
-      atomicAdd(a + 1, acc[r].y);
-      atomicAdd(a + 2, acc[r].z);
-      atomicAdd(a + 3, acc[r].w);
-      atomicAdd(wsum + o, wacc[r]);
-    } else {
-      const float4 a = accum[o];
-      accum[o] = make_float4(a.x + acc[r].x, a.y + acc[r].y, a.z + acc[r].z, a.w + acc[r].w);
-      wsum[o] += wacc[r];
-    }
+    for (int r = 0; r < ROWS; r++) store((group * ROWS + r) * kSplatW + lane, sum[r]);
+    return;
   }
+#pragma unroll
+  for (int r = 0; r < ROWS; r++)
+    for (int c = 0; c < 5; c++) shared.sums.v[c][(group * ROWS + r) * kSplatW + lane] = sum[r][c];
+  const cg::cluster_group tile = cg::this_cluster();
+  tile.sync();
+  // Each block adds up its share of the tile's targets.
+  const int share = kTile / int(gridDim.x);
+  for (int i = int(threadIdx.x); i < share; i += kSplatBlock) {
+    const int t = int(blockIdx.x) * share + i;
+    double v[5] = {};
+    for (uint32_t b = 0; b < gridDim.x; b++) {
+      const SplatSums<ROWS> *s = tile.map_shared_rank(&shared.sums, b);
+      for (int c = 0; c < 5; c++) v[c] += s->v[c][t];
+    }
+    store(t, v);
+  }
+  tile.sync();   // the others read this block's sums
+}
+
+template <int ROWS, bool CLUSTER>
+void launch_splat_tiles(dim3 grid, cudaStream_t st, const JobConsts &jc, uint64_t base, uint32_t n, const float4 *rad,
+                        const float2 *jit, float4 *accum, float *wsum, int ty0, int nrows) {
+  const auto kernel = k_splat<ROWS, CLUSTER>;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = grid.x;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kSplatBlock);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = CLUSTER ? 1 : 0;
+  if (grid.x > 8u) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchKernelEx(&cfg, kernel, jc, base, n, rad, jit, accum, wsum, ty0, nrows);
 }
 
 // The splat of NROWS target rows from TY0 on.
 void launch_splat(const JobConsts &jc, uint64_t base, uint32_t n, const float4 *rad, const float2 *jit,
                   float4 *accum, float *wsum, int ty0, int nrows, cudaStream_t st) {
-  const uint32_t tx = (jc.W + kSplatW - 1) / kSplatW, ty = (uint32_t(nrows) + kSplatH - 1) / kSplatH;
-  // Five blocks fit an SM: split the samples until the blocks fill the device
-  // three times over, which leaves a small last round (853x479 at 9 samples:
-  // 164 us filled once, 145 us three times, 157 us twelve times).
-  const uint64_t tiles = uint64_t(tx) * ty, want = uint64_t(num_sms()) * 5 * 3;
-  uint32_t split = tiles >= want ? 1u : uint32_t(want / tiles);
-  split = split < jc.S ? split : jc.S;
-  const auto kernel = split > 1u ? k_splat<true> : k_splat<false>;
-  kernel<<<dim3(split, tx, ty), 32 * kSplatWarps, 0, st>>>(jc, base, n, rad, jit, accum, wsum, ty0, nrows);
+  const uint32_t across = (jc.W + kSplatW - 1) / kSplatW;
+  auto down = [&](int rows) { return (uint32_t(nrows) + splat_height(rows) - 1) / splat_height(rows); };
+  auto tiles = [&](int rows) { return uint64_t(across) * down(rows); };
+  // Images too small for a block per SM take tiles of a quarter of the height,
+  // whose slices take a third of the time (with k_camera and k_resolve: 64x48 at 64
+  // samples 45 -> 40 us, 20x20 at 1000 356 -> 216; from one to two blocks per SM the
+  // larger tiles are as fast or faster, 200x150 at 4 samples 29 and 33 us).
+  const bool small = tiles(4) * (jc.S < kSplatSplit ? jc.S : kSplatSplit) < uint64_t(num_sms());
+  const int rows = small ? 1 : 4;
+  // Four blocks fit an SM: split the samples while the blocks fill the device no
+  // more than three times over (256x256 at 16 samples 77, 81, 81, 98 us for once,
+  // twice, three, four times, 640x360 at 16 225, 210, 211, 212), among at most the
+  // blocks of a cluster (of 8, the portable size: 64x48 at 64 samples 65 us).
+  const uint64_t want = uint64_t(num_sms()) * 4 * 3;
+  uint32_t split = 1;
+  while (split < kSplatSplit && 2 * split <= jc.S && 2 * split * tiles(rows) <= want) split *= 2;
+  const dim3 grid(split, across, down(rows));
+  const auto launch = small ? (split > 1u ? launch_splat_tiles<1, true> : launch_splat_tiles<1, false>)
+                            : (split > 1u ? launch_splat_tiles<4, true> : launch_splat_tiles<4, false>);
+  launch(grid, st, jc, base, n, rad, jit, accum, wsum, ty0, nrows);
 }
 
 // ImageSampledOutput::set_raw_min_y row flush (image/image-sampled-output.cc:79-123).
