@@ -607,7 +607,9 @@ __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t
       acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
       wacc[r] = 0.f;
     }
-    // A zero weight is skipped where an infinite colour could meet it.
+    // Where a colour is not finite, zero weights are skipped (a weight that the clamp
+    // brings to zero is not: the sample then counts as NaN, as an infinite one
+    // scaled to -0.1 does).
     auto add = [&](auto guard) {
 #pragma unroll 1
       for (int dx = 0; dx < 5; dx++) {
@@ -619,8 +621,9 @@ __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t
 #pragma unroll
           for (int r = 0; r < ROWS; r++) {
             if (h < r || h > r + 4) continue;
-            const float w = fmaxf(ux * sl.wy[h - r][i], lo);
-            if (guard() && w == 0.f) continue;
+            const float product = ux * sl.wy[h - r][i];
+            if (guard() && product == 0.f) continue;
+            const float w = fmaxf(product, lo);
             acc[r].x = fmaf(c.x, w, acc[r].x);
             acc[r].y = fmaf(c.y, w, acc[r].y);
             acc[r].z = fmaf(c.z, w, acc[r].z);
