@@ -535,7 +535,7 @@ union SplatShared {
 // A slice's 25 products per target are summed in 32 bits, and the slices in 64:
 // all products in one 32-bit sum round worse by the square root of the samples
 // (rms of a pixel 3.2e-7 at 16 samples, 6e-7 at 64; 6e-8 so).  The blocks of one
-// tile are a cluster and take every gridDim.x-th sample each; their sums are
+// tile are a cluster and take every SPLIT-th sample each; their sums are
 // added in the order of the blocks, so that an image repeats bit for bit.
 // (Bound by shared-memory latency at 16 warps per SM; at 20 the 64-bit sums do not
 // fit the registers: 1920x1080 at 16 samples 1.64 ms, 2.75 at 20 warps.  Against
@@ -547,14 +547,15 @@ template <int ROWS, bool CLUSTER>
 __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t base, uint32_t n,
                                                           const float4 *__restrict__ rad,
                                                           const float2 *__restrict__ jit, float4 *accum, float *wsum,
-                                                          int ty0, int nrows) {
+                                                          int ty0, int nrows, uint32_t across, uint32_t split) {
   start_after_previous();
   constexpr int kHalo = splat_halo(ROWS), kTile = splat_tile(ROWS);
   __shared__ SplatShared<ROWS> shared;
   SplatSlice<ROWS> &sl = shared.slice;
   const uint32_t p0 = uint32_t(base / jc.S), p1 = uint32_t((base + n) / jc.S);
   const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
-  const int x0 = int(blockIdx.y) * kSplatW, y0 = ty0 + int(blockIdx.z) * splat_height(ROWS);
+  const uint32_t tile_id = blockIdx.x / split, rank = blockIdx.x % split;   // tile, block of the tile
+  const int x0 = int(tile_id % across) * kSplatW, y0 = ty0 + int(tile_id / across) * splat_height(ROWS);
   double sum[ROWS][5] = {};   // colour, alpha, weight
   // This thread's pattern pixels around the tile, from the wave's first on.
   constexpr int kRounds = (kHalo + kSplatBlock - 1) / kSplatBlock;
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t
     const bool in = i < kHalo && pc >= 0 && pc < int(jc.PW) && pr >= 0 && pr < int(jc.PH) && pidx >= p0 && pidx < p1;
     pix[q] = in ? pidx - p0 : ~0u;
   }
-  for (uint32_t k = blockIdx.x; k < jc.S; k += gridDim.x) {
+  for (uint32_t k = rank; k < jc.S; k += split) {
     // All loads of the slice first: their latency is paid once.
     bool wild = false;   // a colour that is not finite
     float2 jq[kRounds];
@@ -577,9 +578,9 @@ __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t
       jq[q] = make_float2(0.f, 0.f);
       rq[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (pix[q] != ~0u) {
-        const size_t at = size_t(pix[q]) * jc.S + k;
-        jq[q] = jit[at];
-        rq[q] = rad[at];
+        const size_t s = size_t(pix[q]) * jc.S + k;
+        jq[q] = jit[s];
+        rq[q] = rad[s];
       }
     }
 #pragma unroll
@@ -664,11 +665,11 @@ __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t
   const cg::cluster_group tile = cg::this_cluster();
   tile.sync();
   // Each block adds up its share of the tile's targets.
-  const int share = kTile / int(gridDim.x);
+  const int share = kTile / int(split);
   for (int i = int(threadIdx.x); i < share; i += kSplatBlock) {
-    const int t = int(blockIdx.x) * share + i;
+    const int t = int(rank) * share + i;
     double v[5] = {};
-    for (uint32_t b = 0; b < gridDim.x; b++) {
+    for (uint32_t b = 0; b < split; b++) {
       const SplatSums<ROWS> *s = tile.map_shared_rank(&shared.sums, b);
       for (int c = 0; c < 5; c++) v[c] += s->v[c][t];
     }
@@ -678,21 +679,22 @@ __global__ void __launch_bounds__(kSplatBlock, 4) k_splat(JobConsts jc, uint64_t
 }
 
 template <int ROWS, bool CLUSTER>
-void launch_splat_tiles(dim3 grid, cudaStream_t st, const JobConsts &jc, uint64_t base, uint32_t n, const float4 *rad,
-                        const float2 *jit, float4 *accum, float *wsum, int ty0, int nrows) {
+void launch_splat_tiles(uint32_t tiles, uint32_t across, uint32_t split, cudaStream_t st, const JobConsts &jc,
+                        uint64_t base, uint32_t n, const float4 *rad, const float2 *jit, float4 *accum, float *wsum,
+                        int ty0, int nrows) {
   const auto kernel = k_splat<ROWS, CLUSTER>;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = grid.x;
+  at.val.clusterDim.x = split;
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
+  cfg.gridDim = dim3(tiles * split);   // one-dimensional: an image may be millions of pixels wide or high
   cfg.blockDim = dim3(kSplatBlock);
   cfg.stream = st;
   cfg.attrs = &at;
   cfg.numAttrs = CLUSTER ? 1 : 0;
-  if (grid.x > 8u) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaLaunchKernelEx(&cfg, kernel, jc, base, n, rad, jit, accum, wsum, ty0, nrows);
+  if (split > 8u) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchKernelEx(&cfg, kernel, jc, base, n, rad, jit, accum, wsum, ty0, nrows, across, split);
 }
 
 // The splat of NROWS target rows from TY0 on.
@@ -714,10 +716,9 @@ void launch_splat(const JobConsts &jc, uint64_t base, uint32_t n, const float4 *
   const uint64_t want = uint64_t(num_sms()) * 4 * 3;
   uint32_t split = 1;
   while (split < kSplatSplit && 2 * split <= jc.S && 2 * split * tiles(rows) <= want) split *= 2;
-  const dim3 grid(split, across, down(rows));
   const auto launch = small ? (split > 1u ? launch_splat_tiles<1, true> : launch_splat_tiles<1, false>)
                             : (split > 1u ? launch_splat_tiles<4, true> : launch_splat_tiles<4, false>);
-  launch(grid, st, jc, base, n, rad, jit, accum, wsum, ty0, nrows);
+  launch(uint32_t(tiles(rows)), across, split, st, jc, base, n, rad, jit, accum, wsum, ty0, nrows);
 }
 
 // ImageSampledOutput::set_raw_min_y row flush (image/image-sampled-output.cc:79-123).
