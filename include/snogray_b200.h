@@ -292,7 +292,9 @@ int snog_trace(SnogScene *scene, const float *rays, uint32_t n, uint32_t n_close
                int32_t *prim, float *t, float *normal, uint64_t *counters4);
 
 /* The same with DEVICE pointers, asynchronous on STREAM (a cudaStream_t,
- * NULL = default stream). */
+ * NULL = default stream).  Calls on different streams may run side by side.  A
+ * captured call keeps 64 bytes of device memory until the scene is destroyed;
+ * two executables of one graph that holds it must not run side by side. */
 int snog_trace_device(SnogScene *scene, const float *d_rays, uint32_t n, uint32_t n_closest,
                       int32_t *d_prim, float *d_t, float *d_normal, void *stream);
 

@@ -310,7 +310,7 @@ int snog_scene_destroy(SnogScene *scene) {
     {
       std::lock_guard<std::mutex> lk(scene->impl->mu);
       if (scene->impl->on_device) device_idle(scene->impl->device);   // traces and renders still running
-      pool_put(scene->impl->trace_scratch);
+      scene->impl->streams.release();
       scene->impl->arena.release();
     }
     delete scene->impl;
@@ -387,10 +387,11 @@ int snog_trace_device(SnogScene *scene, const float *d_rays, uint32_t n, uint32_
     if (!stack_class_for_depth(S.dev.max_depth))
       throw Error{SNOG_EINVAL, "octree deeper than the traversal kernels support (84 levels)"};
     std::lock_guard<std::mutex> lk(S.mu);
-    if (!S.trace_scratch) S.trace_scratch = static_cast<uint32_t *>(pool_get(64));
-    check_cuda(cudaMemsetAsync(S.trace_scratch, 0, 64, cudaStream_t(stream)), "memset");
-    check_cuda(launch_trace_batch(S.dev, d_rays, n, n_closest, d_prim, d_t, d_normal, nullptr,
-                                  S.trace_scratch + 1, S.trace_scratch, cudaStream_t(stream), nullptr),
+    const cudaStream_t st = cudaStream_t(stream);
+    const StreamUses::Call call(S.streams, st);
+    check_cuda(cudaMemsetAsync(call.words(), 0, 4 * StreamUses::kWords, st), "memset");
+    check_cuda(launch_trace_batch(S.dev, d_rays, n, n_closest, d_prim, d_t, d_normal, nullptr, call.words() + 1,
+                                  call.words(), st, nullptr),
                "trace launch");
     return int(SNOG_OK);
   });

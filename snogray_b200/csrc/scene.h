@@ -13,6 +13,7 @@
 #include "device_pool.h"
 #include "octree_build.h"
 #include "snog_common.h"
+#include "stream_use.h"
 #include "wavefront.h"
 
 namespace snog {
@@ -51,7 +52,7 @@ struct SceneImpl {
   // host copies needed by the host side of rendering
   float bbox_min[3], bbox_max[3];
   bool on_device = false;
-  uint32_t *trace_scratch = nullptr;   // ray-batch dispenser counter (+ flags)
+  StreamUses streams;               // of asynchronous ray batches, with their dispenser words
 };
 
 // Working memory of the plain renderer, one per device, shared by every
