@@ -249,6 +249,7 @@ int snog_render_device(SnogScene *scene, const SnogCamera *camera, const SnogRen
     SceneImpl &S = *scene->impl;
     if (!S.on_device) throw Error{SNOG_EINVAL, "scene was built host-only"};
     std::lock_guard<std::mutex> lk(S.mu);
+    const StreamUses::Call call(S.streams, cudaStream_t(stream));
     render_into(S, *camera, *params, d_out_rgb, nullptr, cudaStream_t(stream), stats);
     return int(SNOG_OK);
   });
@@ -308,10 +309,13 @@ int snog_scene_destroy(SnogScene *scene) {
   return guarded([&] {
     if (!scene) return int(SNOG_OK);
     {
-      std::lock_guard<std::mutex> lk(scene->impl->mu);
-      if (scene->impl->on_device) device_idle(scene->impl->device);   // traces and renders still running
-      scene->impl->streams.release();
-      scene->impl->arena.release();
+      SceneImpl &S = *scene->impl;
+      std::lock_guard<std::mutex> lk(S.mu);
+      // Traces and renders may still be running, and an engine's iteration, whose
+      // end is not known here.
+      const bool idle = S.streams.wait() && *S.engines == 0;
+      S.streams.release(idle);
+      S.arena.release(idle);
     }
     delete scene->impl;
     delete scene;

@@ -105,19 +105,20 @@ void pool_put(void *p) {
   P.blocks.erase(it);
 }
 
+void pool_free(void *p) {
+  if (!p) return;
+  {
+    Pool &P = pool();
+    std::lock_guard<std::mutex> lk(P.mu);
+    P.blocks.erase(p);
+  }
+  if (cudaFree(p) != cudaSuccess) cudaGetLastError();
+}
+
 void pool_trim() {
   Pool &P = pool();
   std::lock_guard<std::mutex> lk(P.mu);
   trim_locked(P);
-}
-
-bool device_idle(int device) {
-  int cur = 0;
-  if (cudaGetDevice(&cur) != cudaSuccess) return false;
-  if (cur != device && cudaSetDevice(device) != cudaSuccess) return false;
-  const bool ok = cudaDeviceSynchronize() == cudaSuccess;
-  if (cur != device) cudaSetDevice(cur);
-  return ok;
 }
 
 }  // namespace snog

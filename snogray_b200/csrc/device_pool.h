@@ -25,12 +25,12 @@ void *pool_get(size_t n);
 // this does not wait for the device.
 void pool_put(void *p);
 
+// Free a block of the pool, which waits for the device: for blocks that work may
+// still use, because a wait for it failed or was not made.
+void pool_free(void *p);
+
 // Free every kept block.
 void pool_trim();
-
-// Wait for all work on DEVICE, as cudaFree would have; false if that failed (its
-// blocks are then not to be kept).
-bool device_idle(int device);
 
 }  // namespace snog
 

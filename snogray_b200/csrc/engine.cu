@@ -831,6 +831,7 @@ void Engine::drop_graphs() {
 void Engine::reset_scenes() {
   if (!jobs_.empty()) throw Error{SNOG_EBUSY, "engine has jobs in flight"};
   scenes_.clear();
+  scene_marks_.clear();
 }
 
 void Engine::clear_counters() {
@@ -853,6 +854,8 @@ uint32_t Engine::add_scene(SceneImpl *scene) {
     throw Error{SNOG_EINVAL, "scene has more lights than the engine's max_lights"};
   const uint32_t slot = uint32_t(scenes_.size());
   scenes_.push_back(scene);
+  ++*scene->engines;
+  scene_marks_.emplace_back(nullptr, [n = scene->engines](void *) { --*n; });
   check_cuda(cudaMemcpyAsync(scenes_dev_ + slot, &scene->dev, sizeof(DevScene), cudaMemcpyHostToDevice, stream_),
              "scene table");
   check_cuda(cudaStreamSynchronize(stream_), "scene table");

@@ -251,6 +251,7 @@ class Engine {
   unsigned long long *done_host_ = nullptr;    // pinned
   EngineCtl last_ctl_{};
   std::vector<SceneImpl *> scenes_;
+  std::vector<std::shared_ptr<void>> scene_marks_;   // count this engine in SceneImpl::engines
   std::vector<uint32_t> free_slots_;
   std::deque<uint64_t> pending_;
   std::vector<uint64_t> active_;

@@ -59,6 +59,7 @@ void render_on_engine(SceneImpl &S, const SnogCamera &cam, const SnogRenderParam
   const uint64_t id = e->submit(slot, cam, p, d_out ? d_out : h_out, d_out != nullptr, -1, nullptr, win);
   e->run_to_completion();
   const JobStatsHost js = e->stats(id);
+  e->reset_scenes();   // nothing runs: the scene's memory is not in use here
   if (js.status != SNOG_OK) throw Error{js.status, "render did not complete"};
   if (stats) {
     std::memset(stats, 0, sizeof *stats);
@@ -172,6 +173,7 @@ void render_on(Engine &eng, SnogScene *const *scenes, const SnogCamera *cameras,
     paths += uint64_t(params[i].width) * params[i].height * params[i].spp;
   }
   eng.run_to_completion();
+  eng.reset_scenes();   // nothing runs: the scenes' memory is not in use here
   for (uint32_t i = 0; i < n_jobs; i++)
     if (eng.stats(ids[i]).status != SNOG_OK)
       throw Error{eng.stats(ids[i]).status, "job " + std::to_string(i) + " could not be rendered (device memory)"};

@@ -150,6 +150,7 @@ extern "C" int snog_render_device_noalloc(SnogScene *scene, const SnogCamera *ca
     if (cap > total) cap = total;
 
     std::lock_guard<std::mutex> lk(S.mu);
+    const StreamUses::Call call(S.streams, cudaStream_t(stream));
     char *base = static_cast<char *>(scratch_address());
     float4 *accum = reinterpret_cast<float4 *>(base);
     float *wsum = reinterpret_cast<float *>(base + kMaxPixels * 16);

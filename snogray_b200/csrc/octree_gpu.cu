@@ -410,8 +410,10 @@ struct Scratch {
     return reinterpret_cast<T *>(q);
   }
   ~Scratch() {
-    cudaStreamSynchronize(nullptr);   // the build's stream; a failed build may still be running
-    for (void *q : p) pool_put(q);
+    // The build's stream; a failed build may still be running.
+    const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;
+    if (!idle) cudaGetLastError();
+    for (void *q : p) idle ? pool_put(q) : pool_free(q);
   }
 };
 

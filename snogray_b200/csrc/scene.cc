@@ -45,8 +45,8 @@ void *DeviceArena::upload(const void *src, size_t n) {
   return p;
 }
 
-void DeviceArena::release() {
-  for (void *p : blocks) pool_put(p);
+void DeviceArena::release(bool idle) {
+  for (void *p : blocks) idle ? pool_put(p) : pool_free(p);
   blocks.clear();
   bytes = 0;
 }
@@ -549,8 +549,9 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
       check_cuda(cudaStreamSynchronize(nullptr), "light map guide");
     }
   } catch (...) {
-    device_idle(S.device);
-    A.release();
+    const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;   // the stream of all of the above
+    if (!idle) cudaGetLastError();
+    A.release(idle);
     throw;
   }
   S.on_device = upload;

@@ -3,8 +3,10 @@
 #ifndef SNOG_SCENE_H
 #define SNOG_SCENE_H
 
+#include <atomic>
 #include <cstdint>
 #include <exception>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -35,7 +37,7 @@ struct DeviceArena {
   uint64_t bytes = 0;
   void *alloc(size_t n);           // throws Error on failure
   void *upload(const void *src, size_t n);
-  void release();                  // to the pool: the device must be idle
+  void release(bool idle);         // to the pool if no work can be using them, else freed
 };
 
 struct SceneImpl {
@@ -52,7 +54,9 @@ struct SceneImpl {
   // host copies needed by the host side of rendering
   float bbox_min[3], bbox_max[3];
   bool on_device = false;
-  StreamUses streams;               // of asynchronous ray batches, with their dispenser words
+  StreamUses streams;               // of asynchronous ray batches and renders
+  // Engines whose scene table this scene is in (which may outlive the scene).
+  std::shared_ptr<std::atomic<int>> engines = std::make_shared<std::atomic<int>>(0);
 };
 
 // Working memory of the plain renderer, one per device, shared by every
@@ -99,14 +103,13 @@ void check_cuda(int err, const char *what);   // throws Error{SNOG_ECUDA}
 // RAII device buffer for per-call temporaries (at least 16 bytes, so a
 // zero-length request still yields a valid pointer), from the pool.  The call
 // waits for its work before it returns; one that ends by an exception may not
-// have, and waits here.
+// have, and frees its buffers.
 struct DevBuf {
   void *p = nullptr;
-  int device = 0;
-  explicit DevBuf(size_t n) : p(pool_get(n ? n : 16)) { cudaGetDevice(&device); }
+  explicit DevBuf(size_t n) : p(pool_get(n ? n : 16)) {}
   ~DevBuf() {
-    if (std::uncaught_exceptions()) device_idle(device);
-    pool_put(p);
+    if (std::uncaught_exceptions()) pool_free(p);
+    else pool_put(p);
   }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;

@@ -23,17 +23,15 @@ uint32_t *StreamUses::new_words() {
 StreamUses::Use &StreamUses::find(cudaStream_t st) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   check_cuda(cudaStreamIsCapturing(st, &capture), "stream");
-  const RelaxedCapture relaxed;
   if (capture != cudaStreamCaptureStatusNone) {
-    Use u;
-    u.words = new_words();
-    captured_.push_back(u);
+    captured_.emplace_back();
     return captured_.back();
   }
   unsigned long long id = 0;
   check_cuda(cudaStreamGetId(st, &id), "stream");
   for (Use &u : uses_)
     if (u.stream == id) return u;
+  const RelaxedCapture relaxed;
   for (Use &u : uses_) {
     if (u.lost) continue;
     if (cudaEventQuery(u.done) == cudaSuccess) {
@@ -44,7 +42,6 @@ StreamUses::Use &StreamUses::find(cudaStream_t st) {
   }
   Use u;
   u.stream = id;
-  u.words = new_words();
   check_cuda(cudaEventCreateWithFlags(&u.done, cudaEventDisableTiming), "event");
   uses_.push_back(u);
   return uses_.back();
@@ -57,11 +54,29 @@ StreamUses::Call::~Call() {
   }
 }
 
-void StreamUses::release() {
+uint32_t *StreamUses::Call::words() const {
+  if (!use_.words) {
+    const RelaxedCapture relaxed;
+    use_.words = uses_.new_words();
+  }
+  return use_.words;
+}
+
+bool StreamUses::wait() {
+  bool idle = captured_.empty();
+  for (Use &u : uses_) {
+    const bool ok = !u.lost && cudaEventSynchronize(u.done) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    idle = idle && ok;
+  }
+  return idle;
+}
+
+void StreamUses::release(bool idle) {
   for (Use &u : uses_) cudaEventDestroy(u.done);
   uses_.clear();
   captured_.clear();
-  for (void *p : blocks_) pool_put(p);
+  for (void *p : blocks_) idle ? pool_put(p) : pool_free(p);
   blocks_.clear();
   at_ = nullptr;
   left_ = 0;

@@ -1,5 +1,6 @@
-// stream_use.h -- the streams on which a scene's asynchronous calls run, and a
-// ray-batch dispenser's words for each.
+// stream_use.h -- the streams on which a scene's asynchronous calls run: what has
+// to be waited for before its memory is used for something else, and a ray-batch
+// dispenser's words for each.
 
 #ifndef SNOG_STREAM_USE_H
 #define SNOG_STREAM_USE_H
@@ -21,7 +22,7 @@ class StreamUses {
   struct Use {
     unsigned long long stream = 0;   // the runtime's id, which is not given twice
     cudaEvent_t done = nullptr;      // after the stream's latest call; null for a captured one
-    uint32_t *words = nullptr;
+    uint32_t *words = nullptr;       // allocated when first asked for
     bool lost = false;               // DONE could not be recorded: not for another stream
   };
 
@@ -32,15 +33,22 @@ class StreamUses {
     Use &use_;
     cudaStream_t st_;
 
+    StreamUses &uses_;
+
    public:
-    Call(StreamUses &uses, cudaStream_t st) : use_(uses.find(st)), st_(st) {}
+    Call(StreamUses &uses, cudaStream_t st) : use_(uses.find(st)), st_(st), uses_(uses) {}
     ~Call();
     Call(const Call &) = delete;
     Call &operator=(const Call &) = delete;
-    uint32_t *words() const { return use_.words; }
+    uint32_t *words() const;   // throws Error
   };
-  // Give the words back: no call may be running or captured.
-  void release();
+  // Wait for every call; false if one may still run: a wait failed, or a call
+  // was captured.  (By the streams' events, not for the device, which may not be
+  // waited for while any stream of it is captured.)
+  bool wait();
+  // Give the words back: to the pool if IDLE, that is if no call can be running,
+  // else by freeing them.
+  void release(bool idle);
 
  private:
   std::deque<Use> uses_, captured_;   // (references stay valid)
