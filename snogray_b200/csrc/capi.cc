@@ -183,6 +183,10 @@ static void render_into(SceneImpl &S, const SnogCamera &cam, const SnogRenderPar
   if (e == cudaSuccess) e = cudaEventRecord(pool.done, st);
   if (e == cudaSuccess && !d_out) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
+    // What was launched may be running, on both streams, and no event is behind it.
+    cudaStreamSynchronize(st);
+    if (pool.side.st) cudaStreamSynchronize(pool.side.st);
+    cudaGetLastError();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     throw Error{SNOG_ECUDA, std::string("render: ") + cudaGetErrorString(e)};

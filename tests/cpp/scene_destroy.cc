@@ -10,6 +10,7 @@
 using namespace snog;
 
 static bool launch_fails = false;
+static cudaStream_t shadow_stream = nullptr;   // of the last render
 
 namespace snog {
 int stack_class_for_depth(uint32_t) { return 32; }
@@ -31,9 +32,12 @@ cudaError_t wave_alloc(WaveBuffers &wb, uint64_t cap, uint32_t n_lights) {
   return cudaSuccess;
 }
 cudaError_t render_job(const DevScene &, const JobConsts &, WaveBuffers &, float4 *, float *, float *, cudaStream_t st,
-                       uint32_t *, uint32_t *, RenderProfile *, bool, ShadowStream *) {
+                       uint32_t *, uint32_t *, RenderProfile *, bool, ShadowStream *side) {
+  if (!side->st) cudaStreamCreateWithFlags(&side->st, cudaStreamNonBlocking);
+  shadow_stream = side->st;
   fake::put[st]++;
-  return cudaSuccess;
+  if (launch_fails) fake::put[shadow_stream]++;   // not joined
+  return launch_fails ? cudaErrorInvalidConfiguration : cudaSuccess;
 }
 RenderProfile::~RenderProfile() {}
 }  // namespace snog
@@ -86,6 +90,20 @@ int main() {
     s.destroy();
     fake::expect(fake::completed[stream(24)] == fake::put[stream(24)] || fake::freed.count(s.block),
                  "a render is waited for");
+  }
+  {   // a render that fails half-way
+    Scene s(7 << 20);
+    SnogCamera cam{};
+    SnogRenderParams p{};
+    p.width = p.height = 8;
+    p.spp = 1;
+    float out[3];
+    launch_fails = true;
+    fake::expect(snog_render_device(s.handle, &cam, &p, out, stream(32), nullptr) == SNOG_ECUDA, "render error");
+    launch_fails = false;
+    fake::expect(fake::completed[shadow_stream] == fake::put[shadow_stream], "its shadow rays are waited for");
+    fake::expect(fake::completed[stream(32)] == fake::put[stream(32)], "and the others");
+    s.destroy();
   }
   {
     Scene s(3 << 20);
