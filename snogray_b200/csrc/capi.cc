@@ -158,9 +158,9 @@ static void render_into(SceneImpl &S, const SnogCamera &cam, const SnogRenderPar
     rc.wsum = nullptr;
     rc.out = nullptr;
     rc.npix_cap = 0;
-    check_cuda(cudaMalloc(&rc.accum, npix * sizeof(float4)), "accum");
-    check_cuda(cudaMalloc(&rc.wsum, npix * sizeof(float)), "wsum");
-    check_cuda(cudaMalloc(&rc.out, npix * 3 * sizeof(float)), "out");
+    check_cuda(device_malloc(reinterpret_cast<void **>(&rc.accum), npix * sizeof(float4)), "accum");
+    check_cuda(device_malloc(reinterpret_cast<void **>(&rc.wsum), npix * sizeof(float)), "wsum");
+    check_cuda(device_malloc(reinterpret_cast<void **>(&rc.out), npix * 3 * sizeof(float)), "out");
     rc.npix_cap = npix;
   }
   cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -2,8 +2,6 @@
 
 #include "device_pool.h"
 
-#include <cuda_runtime.h>
-
 #include <map>
 #include <mutex>
 #include <utility>
@@ -119,6 +117,16 @@ void pool_trim() {
   Pool &P = pool();
   std::lock_guard<std::mutex> lk(P.mu);
   trim_locked(P);
+}
+
+cudaError_t device_malloc(void **p, size_t n) {
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    pool_trim();
+    e = cudaMalloc(p, n);
+  }
+  return e;
 }
 
 }  // namespace snog

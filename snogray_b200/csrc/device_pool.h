@@ -4,6 +4,8 @@
 #ifndef SNOG_DEVICE_POOL_H
 #define SNOG_DEVICE_POOL_H
 
+#include <cuda_runtime.h>
+
 #include <cstddef>
 
 namespace snog {
@@ -15,9 +17,8 @@ namespace snog {
 // a scene's creation made fifty of each, a ray batch from host memory five
 // (200k triangles created, traced and destroyed 29 -> 10.6 ms with kept blocks,
 // 300k rays from host memory 3.8 -> 1.2 ms).  Blocks are kept up to kPoolKeep
-// bytes in all and handed out again within a quarter of the size asked for; when
-// an allocation of this library finds the device full they are all freed and
-// it is tried again.
+// bytes, counted over all devices together, and handed out again within a quarter
+// of the size asked for.
 constexpr size_t kPoolKeep = size_t(256) << 20;
 void *pool_get(size_t n);
 
@@ -31,6 +32,10 @@ void pool_free(void *p);
 
 // Free every kept block.
 void pool_trim();
+
+// cudaMalloc for what does not come from the pool: where the device is full, the
+// kept blocks are freed and it is tried again.
+cudaError_t device_malloc(void **p, size_t n);
 
 }  // namespace snog
 

@@ -700,8 +700,7 @@ void *BlockCache::get(size_t n) {
   if (cudaMalloc(&p, r) != cudaSuccess) {
     cudaGetLastError();
     trim();
-    pool_trim();
-    if (cudaMalloc(&p, r) != cudaSuccess) {
+    if (device_malloc(&p, r) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
@@ -761,11 +760,7 @@ Engine::Engine(const EngineConfigHost &cfg, cudaStream_t stream) : cfg_(cfg) {
   size_t o_ctl = take(sizeof(EngineCtl)), o_ring = take(sizeof(WorkItem) * cfg_.ring_items);
   size_t o_jobs = take(sizeof(EngineJobDev) * cfg_.max_jobs), o_done = take(16 * size_t(cfg_.max_jobs));
   size_t o_sc2 = take(sizeof(DevScene) * max_scenes_);
-  if (cudaMalloc(&block_, off) != cudaSuccess) {
-    cudaGetLastError();
-    pool_trim();
-    check_cuda(cudaMalloc(&block_, off), "engine buffers");
-  }
+  check_cuda(device_malloc(&block_, off), "engine buffers");
   char *b = static_cast<char *>(block_);
   for (int k = 0; k < 2; k++) {
     q_o_[k] = reinterpret_cast<float4 *>(b + o_q[k][0]);

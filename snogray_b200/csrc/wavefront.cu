@@ -862,12 +862,7 @@ cudaError_t wave_alloc(WaveBuffers &wb, uint64_t cap, uint32_t n_lights) {
   size_t o_so = take(16 * cap * 2 * nl), o_sd = take(16 * cap * 2 * nl), o_sc = take(16 * cap * 2 * nl);
   size_t o_cnt = take(64), o_stats = take(64);
   char *base = nullptr;
-  cudaError_t e = cudaMalloc(&base, bytes);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    pool_trim();
-    e = cudaMalloc(&base, bytes);
-  }
+  cudaError_t e = device_malloc(reinterpret_cast<void **>(&base), bytes);
   if (e != cudaSuccess) return e;
   wb.block = base;
   wb.bytes = bytes;

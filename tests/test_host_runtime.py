@@ -13,7 +13,7 @@ CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include
 CSRC = os.path.join(ROOT, "snogray_b200", "csrc")
 
 
-@pytest.mark.parametrize("name", ["trace_streams", "scene_destroy"])
+@pytest.mark.parametrize("name", ["trace_streams", "scene_destroy", "full_device"])
 def test_host_code(name, tmp_path):
     gxx = shutil.which("g++")
     if gxx is None:
