@@ -39,46 +39,42 @@ size_t size_class(size_t n) {
   return (n + step - 1) / step * step;
 }
 
-void trim_locked(Pool &P) {
-  for (auto &k : P.kept) {
-    cudaFree(k.second);
-    P.blocks.erase(k.second);
-  }
-  P.kept.clear();
-  P.kept_bytes = 0;
+void free_block(void *p) {
+  if (cudaFree(p) != cudaSuccess) cudaGetLastError();
 }
 
 }  // namespace
+
+// The lock is never held over cudaMalloc or cudaFree, which may wait for the
+// device's work: other threads, of other devices too, need the pool meanwhile.
 
 void *pool_get(size_t n) {
   Pool &P = pool();
   int dev = 0;
   check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-  const size_t want = size_class(n);
-  std::lock_guard<std::mutex> lk(P.mu);
-  auto it = P.kept.lower_bound({dev, want});
-  if (it != P.kept.end() && it->first.first == dev && it->first.second <= want + want / 4) {
-    void *p = it->second;
-    P.kept_bytes -= it->first.second;
-    P.kept.erase(it);
-    return p;
+  size_t size = size_class(n);
+  {
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto it = P.kept.lower_bound({dev, size});
+    if (it != P.kept.end() && it->first.first == dev && it->first.second <= size + size / 4) {
+      void *p = it->second;
+      P.kept_bytes -= it->first.second;
+      P.kept.erase(it);
+      return p;
+    }
   }
   void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, want);
-  if (e == cudaErrorMemoryAllocation && P.kept_bytes) {
-    cudaGetLastError();
-    trim_locked(P);
-    e = cudaMalloc(&p, want);
-  }
+  const cudaError_t e = device_malloc(&p, size);
   if (e != cudaSuccess) {
     cudaGetLastError();
     throw Error{e == cudaErrorMemoryAllocation ? SNOG_ENOMEM : SNOG_ECUDA,
                 std::string("cudaMalloc: ") + cudaGetErrorString(e)};
   }
   try {
-    P.blocks[p] = Block{dev, want};
+    std::lock_guard<std::mutex> lk(P.mu);
+    P.blocks[p] = Block{dev, size};
   } catch (...) {
-    cudaFree(p);
+    free_block(p);
     throw;
   }
   return p;
@@ -87,36 +83,44 @@ void *pool_get(size_t n) {
 void pool_put(void *p) {
   if (!p) return;
   Pool &P = pool();
-  std::lock_guard<std::mutex> lk(P.mu);
-  auto it = P.blocks.find(p);
-  if (it == P.blocks.end()) return;
-  const Block b = it->second;
-  if (P.kept_bytes + b.size <= kPoolKeep) {
-    try {
-      P.kept.insert({{b.device, b.size}, p});
-      P.kept_bytes += b.size;
-      return;
-    } catch (...) {   // no room to remember it: free it
+  {
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto it = P.blocks.find(p);
+    if (it == P.blocks.end()) return;
+    const Block b = it->second;
+    if (P.kept_bytes + b.size <= kPoolKeep) {
+      try {
+        P.kept.insert({{b.device, b.size}, p});
+        P.kept_bytes += b.size;
+        return;
+      } catch (...) {   // no room to remember it: free it
+      }
     }
+    P.blocks.erase(it);
   }
-  cudaFree(p);
-  P.blocks.erase(it);
+  free_block(p);
 }
 
 void pool_free(void *p) {
   if (!p) return;
+  Pool &P = pool();
   {
-    Pool &P = pool();
     std::lock_guard<std::mutex> lk(P.mu);
     P.blocks.erase(p);
   }
-  if (cudaFree(p) != cudaSuccess) cudaGetLastError();
+  free_block(p);
 }
 
 void pool_trim() {
   Pool &P = pool();
-  std::lock_guard<std::mutex> lk(P.mu);
-  trim_locked(P);
+  std::multimap<std::pair<int, size_t>, void *> kept;
+  {
+    std::lock_guard<std::mutex> lk(P.mu);
+    kept.swap(P.kept);
+    P.kept_bytes = 0;
+    for (auto &k : kept) P.blocks.erase(k.second);
+  }
+  for (auto &k : kept) free_block(k.second);
 }
 
 cudaError_t device_malloc(void **p, size_t n) {

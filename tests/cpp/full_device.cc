@@ -6,6 +6,9 @@
 #include "../../snogray_b200/csrc/launch.h"
 #include "../../snogray_b200/csrc/scene.h"
 
+#include <chrono>
+#include <future>
+
 using namespace snog;
 
 namespace snog {
@@ -31,6 +34,7 @@ cudaError_t render_job(const DevScene &, const JobConsts &, WaveBuffers &, float
 RenderProfile::~RenderProfile() {}
 }  // namespace snog
 
+static std::vector<std::future<void>> detached;   // (joined at the end)
 constexpr size_t MiB = size_t(1) << 20;
 
 int main() {
@@ -47,5 +51,29 @@ int main() {
   float out[3];
   fake::expect(snog_render_device(scene, &cam, &p, out, nullptr, nullptr) == SNOG_OK, snog_last_error());
   fake::expect(fake::used < 100 * MiB, "the kept block was freed");
+  // Other threads use the pool while a block is being freed.
+  void *small = pool_get(1 * MiB);
+  pool_put(pool_get(3 * MiB));
+  pool_put(pool_get(30 * MiB));
+  auto others_run = [&](const char *what, auto act) {
+    bool asked = false;
+    fake::on_free = [&] {
+      if (asked) return;
+      asked = true;
+      auto other = std::async(std::launch::async, [&] {
+        pool_put(small);
+        small = pool_get(1 * MiB);
+      });
+      fake::expect(other.wait_for(std::chrono::seconds(2)) == std::future_status::ready, what);
+      detached.push_back(std::move(other));
+    };
+    act();
+    fake::on_free = nullptr;
+    fake::expect(asked, "something was freed");
+  };
+  others_run("the pool is free while it is trimmed", [] { pool_trim(); });
+  fake::capacity = 2048 * MiB;
+  void *large = pool_get(300 * MiB);   // more than is kept
+  others_run("the pool is free while a block is freed", [&] { pool_put(large); });
   return fake::failures != 0;
 }
