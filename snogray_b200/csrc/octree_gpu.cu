@@ -46,6 +46,7 @@
 #include <string>
 #include <vector>
 
+#include "build_scratch.h"
 #include "octree_gpu.h"
 
 namespace snog {
@@ -386,37 +387,6 @@ __global__ void k_scatter_inverse(const uint32_t *perm, uint32_t n, uint32_t *in
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) inv[perm[i]] = i;
 }
 
-// Temporary device memory of one build, given back on every exit path: cut
-// from a few blocks, each twice the one before, of sizes that any build asks
-// the pool for.
-struct Scratch {
-  std::vector<void *> p;
-  char *at = nullptr;
-  size_t left = 0, next = size_t(16) << 20;
-  template <class T>
-  T *get(size_t n) {
-    const size_t need = ((n ? n * sizeof(T) : 16) + 255) & ~size_t(255);
-    if (need > left) {
-      while (next < need) next *= 2;
-      p.reserve(p.size() + 1);
-      at = static_cast<char *>(pool_get(next));
-      p.push_back(at);
-      left = next;
-      next *= 2;
-    }
-    char *q = at;
-    at += need;
-    left -= need;
-    return reinterpret_cast<T *>(q);
-  }
-  ~Scratch() {
-    // The build's stream; a failed build may still be running.
-    const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;
-    if (!idle) cudaGetLastError();
-    for (void *q : p) idle ? pool_put(q) : pool_free(q);
-  }
-};
-
 unsigned grid_for(size_t n) {
   size_t g = (n + 255) / 256;
   if (g < 1) g = 1;
@@ -425,7 +395,7 @@ unsigned grid_for(size_t n) {
 }
 
 template <class T>
-void exclusive_sum(Scratch &S, const T *in, T *out, uint32_t n, cudaStream_t st) {
+void exclusive_sum(BuildScratch &S, const T *in, T *out, uint32_t n, cudaStream_t st) {
   size_t bytes = 0;
   check_cuda(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, st), "scan");
   void *tmp = S.get<unsigned char>(bytes);
@@ -433,7 +403,7 @@ void exclusive_sum(Scratch &S, const T *in, T *out, uint32_t n, cudaStream_t st)
 }
 
 template <class K>
-void sort_pairs(Scratch &S, const K *kin, K *kout, const uint32_t *vin, uint32_t *vout, uint32_t n, int end_bit,
+void sort_pairs(BuildScratch &S, const K *kin, K *kout, const uint32_t *vin, uint32_t *vout, uint32_t n, int end_bit,
                 cudaStream_t st) {
   size_t bytes = 0;
   check_cuda(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kout, vin, vout, n, 0, end_bit, st), "sort");
@@ -455,7 +425,7 @@ void build_octree_device(const MeshArrays &mesh, const std::vector<Box3> &boxes,
                          float4 *prims, DeviceArena &A, DeviceOctree &out) {
   out = DeviceOctree{};
   cudaStream_t st = nullptr;   // legacy stream: ordered with the scene's uploads
-  Scratch S;
+  BuildScratch S;
 
   // ---- 0. the surfaces, in insertion order ---------------------------------
   // (Records and boxes made on the host were most of a scene's creation: 200k
