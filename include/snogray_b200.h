@@ -246,7 +246,8 @@ int snog_ply_free(SnogPlyMesh *mesh);
  * arrays and list order identical to Octree::Builder's); the device builder
  * replays the root's growth on the host and places the surfaces in parallel
  * (octree_gpu.cu).  AUTO, snog_scene_create's choice, uses the device for
- * scenes of 4096 surfaces or more. */
+ * scenes of 4096 surfaces or more, and the host for those that the device
+ * builder does not take or has no memory for. */
 enum { SNOG_OCTREE_AUTO = 0, SNOG_OCTREE_HOST = 1, SNOG_OCTREE_DEVICE = 2 };
 
 /* How the closest-hit traversal deals a node's surface list to the lanes of

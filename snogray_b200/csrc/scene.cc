@@ -45,6 +45,12 @@ void *DeviceArena::upload(const void *src, size_t n) {
   return p;
 }
 
+void DeviceArena::take(DeviceArena &other) {
+  blocks.insert(blocks.end(), other.blocks.begin(), other.blocks.end());
+  bytes += other.bytes;
+  other = DeviceArena{};
+}
+
 void DeviceArena::release(bool idle) {
   for (void *p : blocks) idle ? pool_put(p) : pool_free(p);
   blocks.clear();
@@ -466,15 +472,19 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
     D.prims = d_prims;
     if (dev_oct) {
       try {
+        struct Freed : DeviceArena {   // with the builder's failure
+          ~Freed() { release(false); }
+        } tree;
         build_octree_device(MeshArrays{d.vertices, d.triangles, d.n_vertices, d.n_triangles}, oct_boxes, oct_refs,
-                            d_prims, A, dov);
+                            d_prims, tree, dov);
+        A.take(tree);
         built = true;
       } catch (const Error &e) {
         // Trees the device builder does not take (root grown more than 40
-        // times, deeper than 40 levels, or a descent wider than its stack)
-        // go to the host builder in AUTO mode.  The device builder finds
-        // these before it allocates its outputs in the scene's arena.
-        if (octree_mode != SNOG_OCTREE_AUTO || e.code != SNOG_EINVAL) throw;
+        // times, deeper than 40 levels, or a descent wider than its stack), or
+        // has no room to make on a device that is nearly full, go to the host
+        // builder in AUTO mode.
+        if (octree_mode != SNOG_OCTREE_AUTO || (e.code != SNOG_EINVAL && e.code != SNOG_ENOMEM)) throw;
         std::vector<float4> tri(3 * size_t(d.n_triangles));
         for (uint32_t t = 0; t < d.n_triangles; t++) triangle(t, &tri[3 * size_t(t)]);
         if (!tri.empty())

@@ -37,6 +37,7 @@ struct DeviceArena {
   uint64_t bytes = 0;
   void *alloc(size_t n);           // throws Error on failure
   void *upload(const void *src, size_t n);
+  void take(DeviceArena &other);   // the other's blocks
   void release(bool idle);         // to the pool if no work can be using them, else freed
 };
 
