@@ -556,8 +556,11 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
       };
       D.env_row_guide = guide(D.env_row_cdf, lh, 1, D.row_cells);
       D.env_col_guide = guide(D.env_col_cdf, lw, lh, D.col_cells);
-      check_cuda(cudaStreamSynchronize(nullptr), "light map guide");
     }
+    // A copy from pageable memory returns once it is staged: until here it may
+    // still be on its way to blocks that the scene's destruction hands on, and
+    // that calls on streams of their own read.
+    check_cuda(cudaStreamSynchronize(nullptr), "scene uploads");
   } catch (...) {
     const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;   // the stream of all of the above
     if (!idle) cudaGetLastError();

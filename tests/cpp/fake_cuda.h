@@ -31,6 +31,7 @@ inline int device_waits = 0;         // cudaDeviceSynchronize calls
 inline cudaError_t last = cudaSuccess;
 inline cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
 inline std::function<void()> on_free;
+inline std::function<void(cudaMemcpyKind)> on_copy;   // cudaMemcpy
 inline std::mutex mu;
 
 inline cudaError_t result(cudaError_t e) {
@@ -79,7 +80,10 @@ cudaError_t cudaFree(void *p) {
 }
 cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t st) { fake::put[st]++; return cudaSuccess; }
 cudaError_t cudaMemset(void *, int, size_t) { return cudaSuccess; }
-cudaError_t cudaMemcpy(void *, const void *, size_t, cudaMemcpyKind) { return cudaSuccess; }
+cudaError_t cudaMemcpy(void *, const void *, size_t, cudaMemcpyKind kind) {
+  if (fake::on_copy) fake::on_copy(kind);
+  return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void *, const void *, size_t, cudaMemcpyKind, cudaStream_t st) {
   fake::put[st]++;
   return cudaSuccess;

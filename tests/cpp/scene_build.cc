@@ -65,5 +65,15 @@ int main() {
   fake::expect(snog_scene_create_ex(&d, SNOG_OCTREE_DEVICE, &s) == SNOG_ENOMEM && !s, "DEVICE mode");
   device_error = SNOG_ECUDA;
   fake::expect(snog_scene_create(&d, &s) == SNOG_ECUDA && !s, "other errors");
+  // A copy from pageable memory may return before it has reached the device.
+  fake::on_copy = [](cudaMemcpyKind kind) {
+    fake::put[nullptr]++;
+    if (kind == cudaMemcpyDeviceToHost) fake::complete(nullptr);
+  };
+  for (uint32_t mode : {SNOG_OCTREE_HOST | SNOG_LISTS_SINGLE, SNOG_OCTREE_HOST | SNOG_LISTS_PAIRED}) {
+    fake::expect(snog_scene_create_ex(&d, mode, &s) == SNOG_OK, snog_last_error());
+    fake::expect(fake::completed[nullptr] == fake::put[nullptr], "a new scene's uploads are complete");
+    fake::expect(snog_scene_destroy(s) == SNOG_OK, snog_last_error());
+  }
   return fake::failures != 0;
 }
