@@ -30,7 +30,12 @@ Pool &pool() {
   return *p;
 }
 
-// N rounded up to an eighth of its power of two, at least 4096.
+void free_block(void *p) {
+  if (cudaFree(p) != cudaSuccess) cudaGetLastError();
+}
+
+}  // namespace
+
 size_t size_class(size_t n) {
   if (n <= 4096) return 4096;
   size_t p = 1;
@@ -38,12 +43,6 @@ size_t size_class(size_t n) {
   const size_t step = p / 8;
   return (n + step - 1) / step * step;
 }
-
-void free_block(void *p) {
-  if (cudaFree(p) != cudaSuccess) cudaGetLastError();
-}
-
-}  // namespace
 
 // The lock is never held over cudaMalloc or cudaFree, which may wait for the
 // device's work: other threads, of other devices too, need the pool meanwhile.

@@ -22,6 +22,10 @@ namespace snog {
 constexpr size_t kPoolKeep = size_t(256) << 20;
 void *pool_get(size_t n);
 
+// The size of a block for N bytes: N rounded up to an eighth of its power of two,
+// at least 4096.
+size_t size_class(size_t n);
+
 // Give a block back.  No work that uses it may be running: unlike cudaFree,
 // this does not wait for the device.
 void pool_put(void *p);

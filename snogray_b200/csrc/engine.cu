@@ -680,16 +680,8 @@ void launch_iteration(cudaStream_t st, EngineCtl *ctl, const WorkItem *ring, uin
 
 }  // namespace
 
-size_t BlockCache::round_up(size_t n) {
-  if (n <= 4096) return 4096;
-  size_t p = 1;
-  while (p <= n / 2) p <<= 1;     // largest power of two <= n
-  const size_t step = p / 8;
-  return (n + step - 1) / step * step;
-}
-
 void *BlockCache::get(size_t n) {
-  const size_t r = round_up(n);
+  const size_t r = size_class(n);
   auto it = free_.lower_bound(r);
   if (it != free_.end() && it->first <= r + r / 4) {
     void *p = it->second;

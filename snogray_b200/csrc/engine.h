@@ -96,8 +96,8 @@ struct JobStatsHost {
 };
 
 // Device blocks for per-job buffers, kept for reuse instead of a cudaMalloc
-// and cudaFree per job.  Sizes are rounded up to an eighth of their power of
-// two, so a freed block serves any later request of the same class.
+// and cudaFree per job.  Sizes are those of the pool's blocks (size_class), so a
+// freed block serves any later request of the same class.
 class BlockCache {
  public:
   ~BlockCache() { trim(); }
@@ -107,7 +107,6 @@ class BlockCache {
   uint64_t held() const { return held_; }
 
  private:
-  static size_t round_up(size_t n);
   std::multimap<size_t, void *> free_;
   std::map<void *, size_t> size_of_;
   uint64_t held_ = 0;
