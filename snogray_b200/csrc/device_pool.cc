@@ -2,9 +2,13 @@
 
 #include "device_pool.h"
 
+#include <cstdint>
+#include <iterator>
+#include <list>
 #include <map>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include "scene.h"
 
@@ -17,12 +21,58 @@ struct Block {
   size_t size;
 };
 
+struct Kept {
+  void *p;
+  uint64_t put;   // Pool::puts when it was given back
+};
+
 struct Pool {
   std::mutex mu;
-  std::map<void *, Block> blocks;                           // every block of the pool
-  std::multimap<std::pair<int, size_t>, void *> kept;       // those not in use, by device and size
+  std::map<void *, Block> blocks;                                          // every block of the pool
+  std::list<Kept> kept;                                                    // those not in use, oldest first
+  std::multimap<std::pair<int, size_t>, std::list<Kept>::iterator> find;   // by device and size
   size_t kept_bytes = 0;
+  uint64_t puts = 0;
+
+  // Take the block at IT out of the kept ones.
+  void *take(decltype(find)::iterator it) {
+    void *p = it->second->p;
+    kept_bytes -= it->first.second;
+    kept.erase(it->second);
+    find.erase(it);
+    return p;
+  }
+
+  // Keep P, of B's size.
+  void keep(void *p, const Block &b) {
+    kept.push_back(Kept{p, puts});
+    try {
+      find.insert({{b.device, b.size}, std::prev(kept.end())});
+    } catch (...) {
+      kept.pop_back();
+      throw;
+    }
+    kept_bytes += b.size;
+  }
+
+  // Take the oldest kept block out of the pool.
+  void *drop_oldest() {
+    void *p = kept.front().p;
+    const Block b = blocks.at(p);
+    auto it = find.lower_bound({b.device, b.size});
+    while (it->second != kept.begin()) ++it;
+    take(it);
+    blocks.erase(p);
+    return p;
+  }
 };
+
+// Kept blocks make room for others once so many blocks have been given back since:
+// a scene takes some twenty, so those that scenes or batches of today's sizes use
+// again and again stay, and those of sizes that no longer come go (scenes created
+// after many of 300k triangles, which fill the pool: a 70k-triangle soup 5.1 -> 2.2
+// ms, a terrain of 32k 3.6 -> 1.7, a soup of 6k 1.8 -> 1.15).
+constexpr uint64_t kStale = 256;
 
 // Never destroyed: blocks may be given back while the process ends.
 Pool &pool() {
@@ -54,13 +104,8 @@ void *pool_get(size_t n) {
   size_t size = size_class(n);
   {
     std::lock_guard<std::mutex> lk(P.mu);
-    auto it = P.kept.lower_bound({dev, size});
-    if (it != P.kept.end() && it->first.first == dev && it->first.second <= size + size / 4) {
-      void *p = it->second;
-      P.kept_bytes -= it->first.second;
-      P.kept.erase(it);
-      return p;
-    }
+    auto it = P.find.lower_bound({dev, size});
+    if (it != P.find.end() && it->first.first == dev && it->first.second <= size + size / 4) return P.take(it);
   }
   void *p = nullptr;
   const cudaError_t e = device_malloc(&p, size);
@@ -82,22 +127,28 @@ void *pool_get(size_t n) {
 void pool_put(void *p) {
   if (!p) return;
   Pool &P = pool();
+  std::vector<void *> out;   // blocks to free
   {
     std::lock_guard<std::mutex> lk(P.mu);
     auto it = P.blocks.find(p);
     if (it == P.blocks.end()) return;
     const Block b = it->second;
-    if (P.kept_bytes + b.size <= kPoolKeep) {
-      try {
-        P.kept.insert({{b.device, b.size}, p});
-        P.kept_bytes += b.size;
-        return;
-      } catch (...) {   // no room to remember it: free it
+    P.puts++;
+    try {
+      while (b.size <= kPoolKeep && P.kept_bytes + b.size > kPoolKeep && P.kept.front().put + kStale < P.puts) {
+        out.push_back(nullptr);
+        out.back() = P.drop_oldest();
       }
+      if (P.kept_bytes + b.size <= kPoolKeep) {
+        P.keep(p, b);
+        p = nullptr;
+      }
+    } catch (...) {   // no room to remember it: free it
     }
-    P.blocks.erase(it);
+    if (p) P.blocks.erase(it);
   }
-  free_block(p);
+  for (void *q : out) free_block(q);
+  if (p) free_block(p);
 }
 
 void pool_free(void *p) {
@@ -112,14 +163,15 @@ void pool_free(void *p) {
 
 void pool_trim() {
   Pool &P = pool();
-  std::multimap<std::pair<int, size_t>, void *> kept;
+  std::list<Kept> kept;
   {
     std::lock_guard<std::mutex> lk(P.mu);
     kept.swap(P.kept);
+    P.find.clear();
     P.kept_bytes = 0;
-    for (auto &k : kept) P.blocks.erase(k.second);
+    for (const Kept &k : kept) P.blocks.erase(k.p);
   }
-  for (auto &k : kept) free_block(k.second);
+  for (const Kept &k : kept) free_block(k.p);
 }
 
 cudaError_t device_malloc(void **p, size_t n) {

@@ -18,7 +18,8 @@ namespace snog {
 // (200k triangles created, traced and destroyed 29 -> 10.6 ms with kept blocks,
 // 300k rays from host memory 3.8 -> 1.2 ms).  Blocks are kept up to kPoolKeep
 // bytes, counted over all devices together, and handed out again within a quarter
-// of the size asked for.
+// of the size asked for; where they are full, those not asked for in a long time
+// (kStale) are freed for the next.
 constexpr size_t kPoolKeep = size_t(256) << 20;
 void *pool_get(size_t n);
 

@@ -11,7 +11,7 @@ CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include
 CSRC = os.path.join(os.path.dirname(HERE), "snogray_b200", "csrc")
 
 
-@pytest.mark.parametrize("name", ["build_scratch", "scene_build"])
+@pytest.mark.parametrize("name", ["build_scratch", "scene_build", "pool_sizes"])
 def test_host_memory(name, tmp_path):
     gxx = shutil.which("g++")
     if gxx is None:
