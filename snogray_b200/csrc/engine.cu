@@ -59,7 +59,7 @@ __global__ void k_e_plan(EngineCtl *ctl, const WorkItem *ring, uint32_t R, uint3
   // Retire items fully consumed before this iteration's tickets: their ends
   // increase along the ring, so the first with tickets left is found by
   // bisection (one after the other, the 256 items that fill 16M slots took 92 us
-  // of dependent loads; bisected 9 us, and the terrain frame 164.9 -> 164.3 ms).
+  // of dependent loads; bisected 8 us, and the terrain frame 164.9 -> 164.5 ms).
   unsigned long long head = ctl->item_head, past = ctl->item_tail;
   while (head < past) {
     const unsigned long long mid = head + (past - head) / 2;
@@ -131,9 +131,9 @@ __global__ void __launch_bounds__(256) k_e_regen(EngineCtl *ctl, const WorkItem 
 }
 
 template <int STACK, int PER>
-__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_closest(EngineCtl *ctl, uint32_t cur, const EngineJobDev *jobs,
-                                                      const DevScene *scenes, EQ q, uint32_t *hit_ref,
-                                                      float *hit_t) {
+__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS)
+    k_e_closest(EngineCtl *ctl, uint32_t cur, const EngineJobDev *jobs, const DevScene *scenes, EQ q,
+                uint32_t *hit_ref, float *hit_t) {
   const uint32_t n = ctl->qcount[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->rays_closest += n;
   TraceCounters c{0, 0, 0};
@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_closest
 }
 
 template <int STACK>
-__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_shadow(EngineCtl *ctl, const DevScene *scenes, ESQ q) {
+__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS)
+    k_e_shadow(EngineCtl *ctl, const DevScene *scenes, ESQ q) {
   const uint32_t n = ctl->scount;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->rays_shadow += n;
   TraceCounters c{0, 0, 0};
@@ -178,9 +179,13 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_e_shadow(
 // while many paths are to be traced, free-running blocks of 128 otherwise.
 constexpr int kLongBlock = 896;
 constexpr int shade_blocks(int block) { return block == kLongBlock ? 1 : 6; }   // per SM (72 / 80 registers)
-// Paths left to trace from which the long blocks pay: the engine's terrain
-// renders take 11.43 ms (long: 11.22) at 4.3M paths and 39.8 (38.0) at 17M,
-// Cornell ones 2.73 (2.82) at 1.1M and 34.1 (34.1) at 17M.
+// Paths left to trace from which the long blocks pay.  Whole renders, short / long
+// blocks, at 1.1M, 2.1M, 4.3M and 16.9M paths: Cornell 2.56 / 2.56 ms, 4.39 / 4.43,
+// 8.09 / 8.14, 30.2 / 29.7; mirrors 3.19 / 3.18, 5.70 / 5.56, 10.9 / 10.5, 41.7 / 39.1;
+// a mesh in the open 1.53 / 1.52, 2.18 / 2.12, 3.55 / 3.46, 11.7 / 11.1; far spot lights
+// 1.24 / 1.26, 2.01 / 1.94, 3.61 / 3.31, 12.7 / 10.9; a terrain 3.60 / 3.61, 5.15 / 5.10,
+// 8.32 / 8.26, 27.4 / 26.5; the direct integrator on the Cornell box 2.75 / 2.56, 4.41 /
+// 4.02, 7.72 / 6.95, 28.1 / 23.5.
 constexpr uint64_t kLongPaths = 1u << 21;
 
 // A thread's items of a shading launch over N items are FIRST + k * STRIDE + OFF
@@ -251,11 +256,10 @@ __device__ __forceinline__ uint2 block_append(uint32_t *counts, uint32_t *list0,
 // DIRECT: the direct integrator's code is compiled in (launched while a job
 // of that integrator is active; the path integrator's kernel stays smaller).
 template <bool DIRECT, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, shade_blocks(BLOCK)) k_e_shade(EngineCtl *ctl, uint32_t cur, const EngineJobDev *jobs,
-                                                 const DevScene *scenes, EQ qin, const uint32_t *hit_ref,
-                                                 const float *hit_t, EQ qout, EDL dl,
-                                                 unsigned long long *job_done, unsigned long long *job_spawned,
-                                                 EQ sp, uint32_t sp_cap) {
+__global__ void __launch_bounds__(BLOCK, shade_blocks(BLOCK))
+    k_e_shade(EngineCtl *ctl, uint32_t cur, const EngineJobDev *jobs, const DevScene *scenes, EQ qin,
+              const uint32_t *hit_ref, const float *hit_t, EQ qout, EDL dl, unsigned long long *job_done,
+              unsigned long long *job_spawned, EQ sp, uint32_t sp_cap) {
   const uint32_t n = ctl->qcount[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctl->scount = 0;        // the last iteration's shadow rays are traced: the

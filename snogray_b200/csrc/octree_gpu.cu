@@ -450,7 +450,8 @@ void build_octree_device(const MeshArrays &mesh, const std::vector<Box3> &boxes,
   }
   const uint32_t n = kept + tail;
   if (tail) {
-    check_cuda(cudaMemcpyAsync(d_boxes + kept, boxes.data(), tail * sizeof(Box3), cudaMemcpyHostToDevice, st), "upload");
+    check_cuda(cudaMemcpyAsync(d_boxes + kept, boxes.data(), tail * sizeof(Box3), cudaMemcpyHostToDevice, st),
+               "upload");
     check_cuda(cudaMemcpyAsync(d_refs + kept, refs.data(), tail * 4, cudaMemcpyHostToDevice, st), "upload");
   }
   if (n == 0) {

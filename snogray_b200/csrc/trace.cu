@@ -23,12 +23,11 @@ namespace snog {
 constexpr int batch_blocks(bool count) { return count ? 7 : 8; }
 
 template <int STACK, int PER, bool COUNT>
-__global__ void __launch_bounds__(kTraceBlock, batch_blocks(COUNT)) k_trace_batch(DevScene s, const float *__restrict__ rays,
-                                                     uint32_t n, uint32_t n_closest,
-                                                     int32_t *__restrict__ prim, float *__restrict__ tout,
-                                                     float *__restrict__ nrm,
-                                                     unsigned long long *__restrict__ counters,
-                                                     uint32_t *__restrict__ err, uint32_t *__restrict__ fetch) {
+__global__ void __launch_bounds__(kTraceBlock, batch_blocks(COUNT))
+    k_trace_batch(DevScene s, const float *__restrict__ rays, uint32_t n, uint32_t n_closest,
+                  int32_t *__restrict__ prim, float *__restrict__ tout, float *__restrict__ nrm,
+                  unsigned long long *__restrict__ counters, uint32_t *__restrict__ err,
+                  uint32_t *__restrict__ fetch) {
   unsigned long long cn = 0, ct = 0, an = 0, at = 0;
   TraceCounters c{0, 0, 0}, base{0, 0, 0};
   auto start = [&](uint32_t ray, Traversal<STACK> &tr, bool &any) {
@@ -93,8 +92,6 @@ __global__ void __launch_bounds__(kTraceBlock, batch_blocks(COUNT)) k_trace_batc
   }
 }
 
-// Stack depth needed for a tree of depth D: at most 3 pending entries per
-// level (4 children can pass, one is entered), plus slack.
 // One 48-byte primitive record per surface-list slot, in list order: the
 // record of the slot's primitive id, with the id in c.w (padding slots get a
 // zero record, never read).
@@ -162,6 +159,8 @@ uint32_t probe_pair_lists(const DevScene &s) {
   return cnt[1] > 5 * cnt[0] / 2 ? 1u : 0u;
 }
 
+// Stack depth needed for a tree of depth D: at most 3 pending entries per
+// level (4 children can pass, one is entered), plus slack.
 int stack_class_for_depth(uint32_t depth) {
   uint32_t need = 3 * depth + 4;
   if (need <= 32) return 32;

@@ -13,14 +13,17 @@
 // in the order i = 0,1,2,4,3,5,6,7 (bits swapped so the number of "far" bits
 // never decreases) xor the ray's origin octant, each behind a per-axis gate,
 // and each child call begins with a slab cull.  Here the recursion becomes an
-// explicit stack: all children that pass gate and cull *now* are pushed
-// (at most 4 -- a segment meets at most 4 octants), the first of them is
-// entered directly, and when an entry is popped its gate and cull are
-// evaluated again with the ray's *current* extent.  Because the ray only
-// ever shrinks, the push-time test admits a superset, and the pop-time test
-// is exactly the test the recursion makes at that point; entries are popped
-// in the recursion's order, so the set and order of surface tests -- and the
-// surviving hit -- are the reference's.  The reference's negative-result
+// explicit stack: of the children that pass gate and cull *now* (at most 4 --
+// a segment meets at most 4 octants) the first is entered directly and the
+// others wait in one record; a closest-hit query's next entry is then culled
+// again with the ray's *current* extent.  Because the ray only ever shrinks,
+// the first test admits a superset, and the second decides as the recursion
+// does at that point: with finite bounds whatever the gate closes the cull
+// closes too, so the gate itself is evaluated again only where calls are
+// counted or bounds may be NaN.  (An any-hit query's extent never changes: its
+// entries are not tested again.)  Entries are taken in the recursion's order,
+// so the set and order of surface tests -- and the surviving hit -- are the
+// reference's.  The reference's negative-result
 // cache (space/isec-cache.h) only skips re-testing a surface that already
 // missed; a miss stays a miss for a ray that only shrinks, so omitting it
 // changes work, not results.
@@ -80,8 +83,8 @@ __device__ __forceinline__ bool tripar_hit(float3 corner, float3 e1, float3 e2, 
 // tripar_hit evaluated to the end without early exits: the same
 // operations and the same result, but a warp whose lanes would leave at
 // different tests does not diverge.  What list rounds use (against early exits:
-// the intersection batch +2.4 %; shadow rays of the terrain frame 51.2 -> 50.7
-// ms, of a Cornell render 0.653 -> 0.626).
+// the intersection batch +2.4 %; shadow rays of the terrain frame 51.2 -> 50.6
+// ms, of a Cornell render 0.653 -> 0.623).
 __device__ __forceinline__ bool tripar_hit_flat(float3 corner, float3 e1, float3 e2, bool parallelogram,
                                                 float3 o, float3 d, float t0, float t1, float &t) {
   const float3 pvec = xcross(d, e2);
@@ -272,11 +275,12 @@ __device__ __forceinline__ uint32_t first_child(uint32_t vm) {
 // entry as one call of the reference's recursive function does: parent gate,
 // slab cull, then the node's surface list (left pending in [lp, lend) for
 // list_round) and the children, the first of which -- or else the next child
-// waiting on the stack -- becomes the current entry.  Kernels interleave the steps of many rays per warp and refill
-// lanes whose ray has finished.  The stack holds one record per tree level
-// on the walk's path; kRecs (from STACK, which the host picks from the tree
-// depth) plus kRing records cover every tree the host admits.  Should they
-// not, cnt.overflow is set and the result must be discarded.
+// waiting on the stack -- becomes the current entry.  Kernels interleave the
+// steps of many rays per warp and refill lanes whose ray has finished.  The
+// stack holds one record per tree level on the walk's path; kRecs (from STACK,
+// which the host picks from the tree depth) plus kRing records cover every tree
+// the host admits.  Should they not, cnt.overflow is set and the result must be
+// discarded.
 template <int STACK>
 struct Traversal {
   float3 lo, hi;
@@ -388,8 +392,8 @@ struct Traversal {
   // parent gate, slab cull, then the node's surface list, then its children.
   // Here the qualifying children are pushed when the node is visited and its
   // list is tested afterwards; the push uses the ray's extent before those
-  // tests, which only admits more children (the ray can only shrink), and
-  // every entry's gate and cull are evaluated again when it is entered -- so
+  // tests, which only admits more children (the ray can only shrink), and a
+  // closest-hit query's entries are culled again when they are entered -- so
   // the tests and their order are the reference's.
   // ANY: the queries the calling kernel runs -- kClosestOnly, kAnyOnly or
   // kMixed (checked per ray) -- so closest-hit kernels carry no any-hit branch.

@@ -147,9 +147,9 @@ __device__ __forceinline__ void warp_count(unsigned long long *p, unsigned long 
 // RayDispenser (counters[4]) and interleave one octree entry per ray per
 // iteration, so finished lanes are refilled instead of idling.
 template <int STACK, int PER, bool COUNT>
-__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_closest(DevScene s, RayQ q, uint32_t *counters, uint32_t cur,
-                                                       uint32_t *hit_ref, float *hit_t,
-                                                       unsigned long long *stats) {
+__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS)
+    k_trace_closest(DevScene s, RayQ q, uint32_t *counters, uint32_t cur, uint32_t *hit_ref, float *hit_t,
+                    unsigned long long *stats) {
   start_after_previous();
   const uint32_t n = counters[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_clo
 // Persistent any-hit kernel for the shadow queue (dispenser counters[5]);
 // an unoccluded ray adds its contribution to its path's radiance.
 template <int STACK, bool COUNT>
-__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS) k_trace_shadow(DevScene s, ShadowQ q, uint32_t *counters, float4 *rad,
-                                                      unsigned long long *stats) {
+__global__ void __launch_bounds__(kTraceBlock, SNOG_TRACE_MINBLOCKS)
+    k_trace_shadow(DevScene s, ShadowQ q, uint32_t *counters, float4 *rad, unsigned long long *stats) {
   const uint32_t n = counters[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     stats[1] += n;
