@@ -126,8 +126,10 @@ void OctreeBuilder::insert(uint32_t ref, const Box3 &b, uint32_t node, float x, 
     bool ly = goes_low(b.lo[1], b.hi[1], my, force), hy = goes_high(b.lo[1], b.hi[1], my, force);
     bool lz = goes_low(b.lo[2], b.hi[2], mz, force), hz = goes_high(b.lo[2], b.hi[2], mz, force);
     bool placed = false;
-    // Children are pushed in reverse so they pop in octant order.
-    for (int oc = 7; oc >= 0; oc--) {
+    // Children are pushed in reverse so they pop in octant order.  (A box that
+    // starts on a node's corner and sticks out of it by a rounding error goes to
+    // the corner's child for ever: where halving ends at nothing it stays.)
+    for (int oc = sub > 0 ? 7 : -1; oc >= 0; oc--) {
       bool bx = oc & 4, by = oc & 2, bz = oc & 1;
       if (!((bx ? hx : lx) && (by ? hy : ly) && (bz ? hz : lz))) continue;
       placed = true;
