@@ -557,10 +557,6 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
       D.env_row_guide = guide(D.env_row_cdf, lh, 1, D.row_cells);
       D.env_col_guide = guide(D.env_col_cdf, lw, lh, D.col_cells);
     }
-    // A copy from pageable memory returns once it is staged: until here it may
-    // still be on its way to blocks that the scene's destruction hands on, and
-    // that calls on streams of their own read.
-    check_cuda(cudaStreamSynchronize(nullptr), "scene uploads");
   } catch (...) {
     const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;   // the stream of all of the above
     if (!idle) cudaGetLastError();
@@ -593,10 +589,17 @@ SceneImpl *build_scene(const SnogSceneDesc &d, bool upload, uint32_t octree_mode
   D.horizon = horizon;
   D.max_depth = S.oct.max_depth;
   D.right_handed = d.mesh_right_handed ? 1u : 0u;
-  D.pair_lists = !upload                             ? 0u
-                 : lists_mode == SNOG_LISTS_SINGLE ? 0u
-                 : lists_mode == SNOG_LISTS_PAIRED ? 1u
-                                                   : probe_pair_lists(D);
+  if (upload) try {
+    D.pair_lists = lists_mode == SNOG_LISTS_SINGLE ? 0u : lists_mode == SNOG_LISTS_PAIRED ? 1u : probe_pair_lists(D);
+    // A copy from pageable memory returns once it is staged: until here it may
+    // still be on its way to blocks that the scene's destruction hands on, and
+    // that calls on streams of their own read.  (Waited for after the probe, whose
+    // rays are made meanwhile.)
+    check_cuda(cudaStreamSynchronize(nullptr), "scene uploads");
+  } catch (...) {
+    A.release(false);
+    throw;
+  }
 
   SnogSceneInfo &I = S.info;
   std::memset(&I, 0, sizeof(I));
