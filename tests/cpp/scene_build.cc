@@ -12,10 +12,14 @@
 using namespace snog;
 
 static int device_builds = 0, device_error = SNOG_ENOMEM;
+static bool probe_fails = false;
 
 namespace snog {
 int stack_class_for_depth(uint32_t) { return 32; }
-uint32_t probe_pair_lists(const DevScene &) { return 0; }
+uint32_t probe_pair_lists(const DevScene &) {
+  if (probe_fails) throw Error{SNOG_ECUDA, "list probe"};
+  return 0;
+}
 cudaError_t build_list_records(const uint32_t *, uint32_t, const float4 *, float4 *, cudaStream_t) {
   return cudaSuccess;
 }
@@ -75,5 +79,13 @@ int main() {
     fake::expect(fake::completed[nullptr] == fake::put[nullptr], "a new scene's uploads are complete");
     fake::expect(snog_scene_destroy(s) == SNOG_OK, snog_last_error());
   }
+  fake::on_copy = nullptr;
+  pool_trim();
+  const size_t before = fake::used;
+  probe_fails = true;
+  s = nullptr;
+  fake::expect(snog_scene_create_ex(&d, SNOG_OCTREE_HOST, &s) == SNOG_ECUDA && !s, "a probe that fails");
+  pool_trim();
+  fake::expect(fake::used == before, "its scene's memory is given back");
   return fake::failures != 0;
 }
